@@ -1,23 +1,29 @@
 // cufsp_arnoldi.cu -- the Arnoldi pass of one Krylov step as ONE persistent launch, for generators
-// whose Krylov basis stays in L2 (single-instance solves of 32K-1M states).
+// whose Krylov basis stays on the chip (single-instance solves of 32K-1M states).
 //
 // Same arithmetic contract as the launch sequence of cufsp_krylov.cu (src/KryExpvFSP.cu:38-120,
 // restated there): basis W_k with v_k = rho_k W_k, h = V^T w, w -= V h, ||w||, happy breakdown,
 // ||A v_m||, results in the same device state block.  At these sizes every one of the ~3m kernels
-// of that sequence is latency-bound (a few microseconds of launch and grid-reduction tail each for
-// well under a microsecond of L2 traffic); here one cooperative grid walks all m iterations:
+// of that sequence is latency-bound; here one cooperative grid walks all m iterations.  What bounds an
+// iteration is the chain of waits between CTAs, so the chain is as short as the recurrence allows:
+//  * ONE all-to-all exchange per iteration.  The norm of W_j is not waited for before A W_j is formed:
+//    each CTA publishes its partial sums of ||W_j||^2 together with those of W_k . (A W_j), k <= j, and
+//      rho_j = 1/||W_j||,  h_k = rho_k rho_j W_k . (A W_j),  W_{j+1} = rho_j (A W_j - sum_k rho_k^2 (W_k . A W_j) W_k)
+//    follow from the totals: the same quantities as with a normalisation first, to rounding.  The
+//    breakdown test of W_j then runs one iteration later, after one generator application too many.
+//  * no grid barrier (cufsp_grid.cuh): partial sums and the entries of W_j that other CTAs gather are
+//    polled as data.  Every CTA sums the partials in the same fixed order, so all take identical
+//    decisions.
 //  * the generator is applied from a per-state term table built once per coefficient vector:
 //      (A x)[i] = sum_t coef[t][i] x[i - shift_t]   (last term: shift 0, the diagonal),
-//    coefficient 0 wherever the source state leaves the box (its index is clamped to [0, n)), so
-//    the gather needs no multi-index decode; the same form holds for A^T (adjoint solves);
-//  * the dot products h = V^T w are taken in the same pass that produces w = rho_j A W_j (each
-//    thread owns its states for the whole launch, so its w values need no barrier);
-//  * two grid barriers per iteration (after the dots, after the norm); each barrier completes a
-//    deterministic reduction: every CTA writes its partial sums, and after the barrier EVERY CTA
-//    sums all partials in the same fixed order, so all CTAs take identical decisions;
-//  * barrier waits are bounded (~0.3 s); on expiry the kernel sets an error word, every CTA leaves
-//    at its next barrier, and the host reports CUFSP_ERR_CUDA.  The launch is cooperative, so all
-//    CTAs are co-resident.
+//    coefficient 0 wherever the source state leaves the box (its index is clamped to [0, n)).  A CTA
+//    owns a contiguous slice of the states; up to 2 states per thread and 12 terms the coefficients stay
+//    in registers for the whole launch, and sources inside the slice come from shared memory.
+//  * the CTA's slices of as many basis vectors as fit live in shared memory (all 30 of them up to 148 x
+//    ~890 = 131K states); the dots and the update read them there and the rest from L2.
+// Measured, one pass of m = 30 (events around the launch): @PASS@
+// Waits are bounded; on expiry the kernel sets an error word, every CTA leaves, and the host reports
+// CUFSP_ERR_CUDA.  The launch is cooperative, so all CTAs are co-resident.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -27,23 +33,29 @@
 #include <mutex>
 
 #include "cufsp_internal.h"
+#include "cufsp_grid.cuh"
 
 namespace cufsp {
 
 namespace {
 
-constexpr int kPThreads = 1024;
-constexpr int kPWarps = kPThreads / 32;
-constexpr int kKMax = 64;            // partial sums per CTA (>= CUFSP_MAX_KRYLOV)
 constexpr int kMaxTerms = 64;
-constexpr unsigned long long kWaitNs = 300ull * 1000 * 1000;  // a grid barrier gives up after 0.3 s
+constexpr int kHaloMax = 64;   // largest |shift| of a term whose sources are read from shared memory
+constexpr int kMaxNear = 10, kMaxFar = 8;
+constexpr int kPThreadsMax = 512;
+constexpr int kPWarpsMax = kPThreadsMax / 32;
 
 struct PArgs {
-    int64_t n;
-    int64_t chunk;              // states per CTA (the last CTA may have fewer)
+    int n;
+    int chunk;                  // states per CTA, even (the last CTA may have fewer)
+    int slots;                  // basis vectors whose slices live in shared memory
+    int ring;                   // > 0: W_k is in slot k % ring (incomplete orthogonalisation); 0: W_k in slot k < slots
     int T;
     const double *coef;         // [T][n]
-    int64_t shift[kMaxTerms];   // source index i - shift[t] (clamped)
+    int shift[kMaxTerms];       // source index i - shift[t] (clamped)
+    // register variants: the terms with |shift| <= halo, and the others (term, -1: none)
+    int n_near, n_far, halo;
+    short near_t[kMaxNear], far_t[kMaxFar];
     const double *v0;           // W_0 (the caller's vector)
     double *W;                  // W_1 .. W_{m+1}
     double *H, *rho, *gam, *beta, *avnorm;
@@ -51,234 +63,363 @@ struct PArgs {
     int mp2, m, iop, q;
     double btol;
     int with_avnorm;
-    double *part;               // [2][kKMax][gridDim.x] (k-major)
-    unsigned *bar;              // arrival counter, zero at launch
-    int *err;                   // set when a barrier wait expired
+    double *ex;                 // exchange area of this launch, all unset
+    double *ex_next;            // that of the next launch, set back to unset here
+    int ex_rows;                // rows of an area
+    int *err;                   // set when a wait expired
 };
 
 struct PSmem {
-    double wsum[kPWarps];
-    double res[kKMax];
-    double rho[CUFSP_MAX_KRYLOV + 2];
-    double gam[kKMax];
-    int ok;
+    double2 c2[(CUFSP_MAX_KRYLOV + 4) / 2];  // c_r = rho_k^2 W_k . (A W_j) of the vector at position r; 0 for W_j
+    double part[kPWarpsMax][4];              // dots of one warp's four vectors over its part of the slice
+    double wsum[kPWarpsMax], asum[kPWarpsMax];  // per-warp sums of ||W_j||^2 and of ||A W_m||^2
+    double dot[CUFSP_MAX_KRYLOV + 2];        // W_k . (A W_j) by position
+    double rho[CUFSP_MAX_KRYLOV + 2];        // by k
+    double sn, rj;                           // ||W_j||, 1 / ||W_j||
 };
 
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-__device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-// Grid barrier number `epoch` (1, 2, ...): the arrival counter reaches epoch * gridDim.x.
-__device__ __forceinline__ bool grid_sync(const PArgs &a, unsigned &epoch, int &ok_s) {
-    __syncthreads();
-    ++epoch;
-    if (threadIdx.x == 0) {
-        // arrival with release semantics (the CTA's partial sums and w become visible first), then a
-        // tight acquire poll; a measured cooperative probe: 1.26 us per barrier over 148 CTAs, against
-        // 1.39-1.64 us for a fence, a relaxed atomic and 64 ns sleeps between polls.  The wait is
-        // bounded by the global timer (kWaitNs); the error word is looked at every 64 polls.
-        asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(a.bar), "r"(1u) : "memory");
-        const unsigned target = epoch * gridDim.x;
-        int ok = 1;
-        const unsigned long long t0 = global_ns();
-        for (int it = 1; ld_acquire(a.bar) < target; ++it) {
-            if ((it & 63) == 0) {
-                if (*(volatile int *)a.err) {  // another CTA gave up
-                    ok = 0;
-                    break;
-                }
-                if (global_ns() - t0 > kWaitNs) {
-                    atomicExch(a.err, 1);
-                    ok = 0;
-                    break;
-                }
-            }
-        }
-        __threadfence();
-        ok_s = ok && *(volatile int *)a.err == 0;
-    }
-    __syncthreads();
-    return ok_s != 0;
-}
-
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-// Grid totals of the K per-CTA partials already stored in part[0..K)[blockIdx.x] (k-major) into
-// sm.res, identical in every CTA: all threads copy the K x G partials into shared memory in one
-// coalesced pass, then one warp per k sums them in a fixed order.  False when a barrier wait expired.
-__device__ __forceinline__ bool finish_reduce(int K, const double *part, double *red, PSmem &sm, const PArgs &a,
-                                              unsigned &epoch) {
-    if (!grid_sync(a, epoch, sm.ok)) return false;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int G = gridDim.x;
-    for (int p = threadIdx.x; p < K * G; p += blockDim.x) red[p] = __ldcg(part + p);
-    __syncthreads();
-    for (int k = warp; k < K; k += kPWarps) {
-        double v = 0.0;
-        for (int b = lane; b < G; b += 32) v += red[k * G + b];
-        v = warp_sum(v);
-        if (lane == 0) sm.res[k] = v;
-    }
-    __syncthreads();
-    return true;
-}
-
-// Block sum of one value per thread into part[0][blockIdx.x] (fixed order), then finish_reduce.
-__device__ __forceinline__ bool reduce1(double v, double *part, double *red, PSmem &sm, const PArgs &a,
-                                        unsigned &epoch) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    v = warp_sum(v);
-    if (lane == 0) sm.wsum[warp] = v;
-    __syncthreads();
-    if (warp == 0) {
-        double t = warp_sum(sm.wsum[lane]);
-        if (lane == 0) __stcg(part + blockIdx.x, t);
-    }
-    return finish_reduce(1, part, red, sm, a, epoch);
-}
-
-// (A x)[i] from the term table (one state).
-__device__ __forceinline__ double term_apply(const PArgs &a, const double *x, int64_t i) {
-    double s = 0.0;
-    for (int t = 0; t < a.T; ++t) {
-        int64_t src = i - a.shift[t];
-        src = src < 0 ? 0 : (src >= a.n ? a.n - 1 : src);
-        s = fma(__ldg(a.coef + (size_t)t * a.n + i), __ldcg(x + src), s);
-    }
-    return s;
-}
-
-// CTA b owns the states [b chunk, (b + 1) chunk); its slice of the newest vector w lives in shared
-// memory (ws) as well as in global memory (for the other CTAs' neighbour gathers).
-__global__ void __launch_bounds__(kPThreads, 1) k_arnoldi_persistent(const PArgs a) {
-    extern __shared__ double ws[];  // [chunk] own slice of w, then [m][gridDim.x] partial sums
-    __shared__ PSmem sm;
-    const int64_t n = a.n;
-    const int64_t lo = (int64_t)blockIdx.x * a.chunk;
-    const int len = (int)max((int64_t)0, min(a.chunk, n - lo));
+// NT threads.  TN > 0: at most NS states per thread, TN near and TF far terms, coefficients in registers;
+// the near terms' sources come from the slice in shared memory, extended on both sides by a halo of the
+// neighbours' entries, the far terms' from L2, all loads of a thread in flight together.  TN = 0: any.
+// 8 warps with up to 4 states per thread rather than 16 or 32 with fewer: at these sizes the instructions
+// that every warp spends on addresses, reductions and waits, not the data, fill an iteration between two
+// waits, and a thread of 8 warps has 255 registers, so that nothing spills (a spill goes to L2: shared
+// memory leaves little L1).
+template <int NT, int NS, int TN, int TF>
+__global__ void __launch_bounds__(NT, 1) k_arnoldi_persistent(const __grid_constant__ PArgs a) {
+    extern __shared__ __align__(16) double ws[];  // [chunk] slice of A W_j | [halo][chunk][halo] of W_j | [slots][chunk] basis
+    __shared__ __align__(16) PSmem sm;
+    constexpr bool REG = TN > 0;
+    constexpr int NW = NT / 32, LNW = NW == 16 ? 4 : 3;
+    static_assert(NW == 1 << LNW, "8 or 16 warps");
+    const int lo = (int)blockIdx.x * a.chunk;
+    const int len = min(a.chunk, a.n - lo);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool lead = blockIdx.x == 0 && tid == 0;
-    const int mp2 = a.mp2;
-    unsigned epoch = 0;
-    int rc = 0;
-    auto part = [&]() { return a.part + (size_t)((rc++) & 1) * gridDim.x * kKMax; };
-    auto wv = [&](int k) -> const double * { return k == 0 ? a.v0 : a.W + (size_t)(k - 1) * n; };
-    double *red = ws + a.chunk;
+    double *const xs = ws + a.chunk + a.halo;
+    double *const slot0 = xs + a.chunk + a.halo;
+    double *const c = reinterpret_cast<double *>(sm.c2);
+    const int pitch = exchange_pitch((int)gridDim.x);
 
+#pragma unroll 1
+    for (int p = (int)blockIdx.x * NT + tid; p < exchange_doubles(a.ex_rows, (int)gridDim.x); p += (int)gridDim.x * NT)
+        a.ex_next[p] = unset_value();
     if (blockIdx.x == 0) {
-        for (int i = tid; i < mp2 * mp2; i += blockDim.x) a.H[i] = 0.0;
-        for (int i = tid; i < mp2; i += blockDim.x) {
-            a.rho[i] = 0.0;
-            a.gam[i] = 0.0;
+#pragma unroll 1
+        for (int i = tid; i < a.mp2 * (a.mp2 + 2); i += NT) a.H[i] = 0.0;  // H, rho and gam are contiguous
+    }
+#pragma unroll 1
+    for (int il = tid; il < (a.slots + 2) * a.chunk + 2 * a.halo; il += NT) ws[il] = 0.0;
+    if (tid < CUFSP_MAX_KRYLOV + 4) c[tid] = 0.0;  // positions a loop rounded up to four may read
+    __syncthreads();
+    double cn[NS][REG ? TN : 1], cfar[NS][REG ? TF : 1];
+    if constexpr (REG) {
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            const int il = tid + s * NT;
+            const double *cp = a.coef + lo + il;
+#pragma unroll
+            for (int t = 0; t < TN; ++t) cn[s][t] = t < a.n_near && il < len ? __ldcg(cp + (size_t)a.near_t[t] * a.n) : 0.0;
+#pragma unroll
+            for (int t = 0; t < TF; ++t) cfar[s][t] = t < a.n_far && il < len ? __ldcg(cp + (size_t)a.far_t[t] * a.n) : 0.0;
         }
     }
     double acc = 0.0;
-    for (int il = tid; il < len; il += blockDim.x) {
+#pragma unroll 1
+    for (int il = tid; il < len; il += NT) {
         const double t = __ldcg(a.v0 + lo + il);
+        xs[il] = t;
+        if (a.slots > 0) slot0[il] = t;
         acc = fma(t, t, acc);
+        double *w = a.W + lo + il;
+#pragma unroll 2
+        for (int k = 0; k < a.m; ++k, w += a.n) st_relaxed(w, unset_value());
     }
-    if (!reduce1(acc, part(), red, sm, a, epoch)) return;
-    const double beta = sqrt(sm.res[0]);
-    const int flag0 = !isfinite(beta) ? -1 : (beta == 0.0 ? -2 : 0);
-    if (tid == 0) sm.rho[0] = beta > 0.0 ? 1.0 / beta : 0.0;
-    __syncthreads();  // block 0's clearing of rho/gam precedes the writes below
-    if (lead) {
-        *a.beta = beta;
-        *a.avnorm = 0.0;
-        a.rho[0] = sm.rho[0];
-        *a.flag = flag0;
-    }
-    if (flag0) return;
+    acc = warp_sum(acc);
+    if (lane == 0) sm.wsum[warp] = acc;
+    __syncthreads();
 
-    for (int j = 0; j < a.m; ++j) {
+    int pj = 0;                // position of W_j in its window
+    int row = 0;               // first exchange row of this iteration
+    const double *x = a.v0;    // W_j
+#pragma unroll 1
+    for (int j = 0;; ++j) {
+        const bool last = j == a.m;
         const int istart = a.iop ? max(0, j - a.q + 1) : 0;
-        const int K = j - istart + 1;
-        const double *x = wv(j);
-        double *w = a.W + (size_t)j * n;  // W_{j+1}
-        const double rj = sm.rho[j];
-        // w = rho_j A W_j on the own slice
-        for (int il = tid; il < len; il += blockDim.x) {
-            const double wi = rj * term_apply(a, x, lo + il);
-            ws[il] = wi;
-            __stcg(w + lo + il, wi);
+        const int K = last ? 0 : j - istart + 1;
+        const int rows = last ? 1 + a.with_avnorm : K + 1;
+        const int Kres = a.ring > 0 ? K : max(0, min(K, a.slots - istart));  // positions in shared memory
+        const double *const base = slot0 + (a.ring > 0 ? 0 : istart * a.chunk);
+        const double *const gbase = a.W + lo + ((long long)istart - 1) * a.n;   // position r > 0: + r n
+        double *const mine = a.ex + (size_t)row * pitch + blockIdx.x;
+        double w[NS];
+        double aw2 = 0.0;
+        Patience wait;
+        bool bad = false;
+        if (warp == NW - 1 && j > 0) {  // row 0: ||W_j||^2, on its way while A W_j is formed
+            const double v = warp_sum(lane < NW ? sm.wsum[lane] : 0.0);
+            if (lane == 0) st_relaxed(mine, settled(v));
+        }
+        // entry rel of the slice from L2 (unset until its owner has stored it)
+        auto far = [&](int rel) -> double { return ld_relaxed(x + min(max(lo + rel, 0), a.n - 1)); };
+        if (!last || a.with_avnorm) {
+            if constexpr (REG) {
+                double v[NS][TF];
+#pragma unroll
+                for (int s = 0; s < NS; ++s)
+#pragma unroll
+                    for (int t = 0; t < TF; ++t) {
+                        v[s][t] = 0.0;
+                        if (t < a.n_far && s * NT < len) v[s][t] = far(tid + s * NT - a.shift[a.far_t[t]]);
+                    }
+                if (tid < 2 * a.halo) {
+                    const int rel = tid < a.halo ? tid - a.halo : len + tid - a.halo;
+                    double h = far(rel);
+                    while (j > 0 && is_unset(h)) {
+                        if (wait.give_up(a.err)) {
+                            bad = true;
+                            break;
+                        }
+                        h = far(rel);
+                    }
+                    xs[rel] = h;
+                }
+                __syncthreads();
+#pragma unroll
+                for (int s = 0; s < NS; ++s) w[s] = 0.0;
+#pragma unroll
+                for (int t = 0; t < TN; ++t) {
+                    if (t >= a.n_near) break;
+                    const double *p = xs + tid - a.shift[a.near_t[t]];
+#pragma unroll
+                    for (int s = 0; s < NS; ++s)
+                        if (tid + s * NT < len) w[s] = fma(cn[s][t], p[s * NT], w[s]);
+                }
+                if (j > 0) {
+                    for (;;) {
+                        bool miss = false;
+#pragma unroll
+                        for (int s = 0; s < NS; ++s)
+#pragma unroll
+                            for (int t = 0; t < TF; ++t)
+                                if (is_unset(v[s][t])) {
+                                    miss = true;
+                                    v[s][t] = far(tid + s * NT - a.shift[a.far_t[t]]);
+                                }
+                        if (!miss) break;
+                        if (wait.give_up(a.err)) {
+                            bad = true;
+                            break;
+                        }
+                    }
+                }
+#pragma unroll
+                for (int s = 0; s < NS; ++s) {
+#pragma unroll
+                    for (int t = 0; t < TF; ++t) w[s] = fma(cfar[s][t], v[s][t], w[s]);
+                    if (tid + s * NT < len) ws[tid + s * NT] = w[s];
+                    else w[s] = 0.0;
+                    aw2 = fma(w[s], w[s], aw2);
+                }
+            } else {
+#pragma unroll 1
+                for (int il = tid; il < len; il += NT) {
+                    double sum;
+                    bool miss;
+                    do {
+                        sum = 0.0;
+                        miss = false;
+#pragma unroll 4
+                        for (int t = 0; t < a.T; ++t) {
+                            const int rel = il - a.shift[t];
+                            double v;
+                            if ((unsigned)rel < (unsigned)len) v = xs[rel];
+                            else v = far(rel);
+                            miss = miss || is_unset(v);
+                            sum = fma(__ldg(a.coef + (size_t)t * a.n + lo + il), v, sum);
+                        }
+                        if (j == 0 || !miss) break;
+                        bad = bad || wait.give_up(a.err);
+                    } while (!bad);
+                    ws[il] = sum;
+                    aw2 = fma(sum, sum, aw2);
+                }
+            }
+        }
+        if (last) {
+            aw2 = warp_sum(aw2);
+            if (lane == 0) sm.asum[warp] = aw2;
+        }
+        if (__syncthreads_or(bad)) return;
+        // dots over the slice: a warp takes four positions and one part of the slice, so that each entry
+        // of A W_j is read once for four products
+        const int lnb = K > 32 ? 4 : K > 16 ? 3 : K > 8 ? 2 : K > 4 ? 1 : 0, nb = 1 << lnb;
+        const int nsl = NW >> lnb;  // parts (0: more groups of four than warps)
+#pragma unroll 1
+        for (int r0 = (warp & (nb - 1)) * 4, part = warp; r0 < K; r0 += 4 * NW, part += NW) {
+            const int half = a.chunk >> 1, per = nsl > 1 ? (half + nsl - 1) >> (LNW - lnb) : half;
+            const int b0 = nsl > 1 ? (warp >> lnb) * per : 0, b1 = min(half, b0 + per);
+            const int q1 = min(r0 + 1, K - 1), q2 = min(r0 + 2, K - 1), q3 = min(r0 + 3, K - 1);
+            double d0 = 0.0, d1 = 0.0, d2 = 0.0, d3 = 0.0;
+            if (q3 < Kres) {
+                const double2 *p0 = reinterpret_cast<const double2 *>(base + r0 * a.chunk);
+                const double2 *p1 = reinterpret_cast<const double2 *>(base + q1 * a.chunk);
+                const double2 *p2 = reinterpret_cast<const double2 *>(base + q2 * a.chunk);
+                const double2 *p3 = reinterpret_cast<const double2 *>(base + q3 * a.chunk);
+                const double2 *pw = reinterpret_cast<const double2 *>(ws);
+#pragma unroll 2
+                for (int b = b0 + lane; b < b1; b += 32) {
+                    const double2 u = pw[b], u0 = p0[b], u1 = p1[b], u2 = p2[b], u3 = p3[b];
+                    d0 = fma(u0.y, u.y, fma(u0.x, u.x, d0));
+                    d1 = fma(u1.y, u.y, fma(u1.x, u.x, d1));
+                    d2 = fma(u2.y, u.y, fma(u2.x, u.x, d2));
+                    d3 = fma(u3.y, u.y, fma(u3.x, u.x, d3));
+                }
+            } else {
+                const double *p0 = istart + r0 == 0 ? a.v0 + lo : gbase + (size_t)r0 * a.n;
+                const double *p1 = gbase + (size_t)q1 * a.n, *p2 = gbase + (size_t)q2 * a.n, *p3 = gbase + (size_t)q3 * a.n;
+                if (istart + q1 == 0) p1 = p2 = p3 = p0;  // K = 1
+#pragma unroll 4
+                for (int il = 2 * b0 + lane; il < min(len, 2 * b1); il += 32) {
+                    const double u = ws[il];
+                    d0 = fma(__ldcg(p0 + il), u, d0);
+                    d1 = fma(__ldcg(p1 + il), u, d1);
+                    d2 = fma(__ldcg(p2 + il), u, d2);
+                    d3 = fma(__ldcg(p3 + il), u, d3);
+                }
+            }
+            d0 = warp_sum4(d0, d1, d2, d3);
+            if ((lane & 7) == 0) sm.part[part][lane >> 3] = d0;
         }
         __syncthreads();
-        // h_k partials: one warp per basis vector, w from shared memory
-        {
-            double *pp = part();
-            for (int k = warp; k < K; k += kPWarps) {
-                const double *vk = wv(istart + k) + lo;
-                double d = 0.0;
-                for (int il = lane; il < len; il += 32) d = fma(__ldcg(vk + il), ws[il], d);
-                d = warp_sum(d);
-                if (lane == 0) __stcg(pp + (size_t)k * gridDim.x + blockIdx.x, d);
-            }
-            if (!finish_reduce(K, pp, red, sm, a, epoch)) return;
-        }
+        // publish the other rows: the dots, or ||A W_m||^2
+        if (j == 0) __threadfence();  // the cleared basis is visible before any CTA passes this exchange
         if (tid < K) {
-            const int kk = istart + tid;
-            const double r = sm.rho[kk];
-            const double h = r * sm.res[tid];
-            sm.gam[tid] = h * r;
-            if (blockIdx.x == 0) {
-                a.H[kk + (size_t)j * mp2] = h;
-                a.gam[kk] = h * r;
+            double v = sm.part[tid >> 2][tid & 3];
+#pragma unroll 4
+            for (int u = 1; u < nsl; ++u) v += sm.part[(u << lnb) + (tid >> 2)][tid & 3];
+            st_relaxed(mine + (size_t)(1 + tid) * pitch, settled(v));
+        }
+        if (warp == NW - 1 && (last || j == 0)) {
+            const double v = warp_sum(lane < NW ? (last ? sm.asum : sm.wsum)[lane] : 0.0);
+            if (lane == 0 && (j == 0 || rows == 2)) st_relaxed(mine + (j == 0 ? 0 : pitch), settled(v));
+        }
+        if (!exchange_own(a.ex, a.ex_rows, row, rows, 1, NW, j == 0, a.err)) bad = true;
+        if (warp == 0) {
+#pragma unroll 1
+            for (int r = lane + 1; r < rows; r += 32) {
+                const int pos = r - 1;
+                const int k = a.ring > 0 ? pos + a.ring * ((j - pos) / a.ring) : istart + pos;
+                const double rk = k < j ? sm.rho[k] : 0.0;
+                double v;
+                if (!exchange_total(a.ex, a.ex_rows, row, r, a.err, v)) bad = true;
+                sm.dot[pos] = v;
+                c[pos] = v * (rk * rk);
+            }
+        } else if (warp == NW - 1) {  // the norm has come earlier: its root and inverse hide behind the dots
+            double v;
+            if (!exchange_total(a.ex, a.ex_rows, row, 0, a.err, v)) bad = true;
+            const double sn = sqrt(v);
+            sm.sn = sn;
+            sm.rj = sn > 0.0 ? 1.0 / sn : 0.0;
+        }
+        if (j == 0) __threadfence();
+        if (__syncthreads_or(bad)) return;
+        row += rows;
+        const double sn = sm.sn, rj = sm.rj;
+        // 0: go on, else the flag that ends the pass: happy breakdown (src/KryExpvFSP.cu:90-98) at W_j
+        const int stop = !isfinite(sn) ? -1 : j == 0 ? (sn == 0.0 ? -2 : 0) : (sn < a.btol ? j : 0);
+        if (stop || last) {
+            if (lead) {
+                if (j == 0) {
+                    *a.beta = sn;
+                    *a.avnorm = 0.0;
+                    a.rho[0] = rj;
+                }
+                *a.flag = stop;
+                if (last && !stop) {
+                    a.H[j + (j - 1) * a.mp2] = sn;
+                    a.rho[j] = rj;
+                    if (rows == 2) {  // ||A v_m|| (src/KryExpvFSP.cu:114-120)
+                        const double av = rj * sqrt(sm.dot[0]);
+                        *a.avnorm = av;
+                        if (!isfinite(av)) *a.flag = -1;
+                    }
+                }
+            }
+            return;
+        }
+        // W_{j+1} = rho_j (A W_j - sum_k c_k W_k), and its squared norm
+        const double cj = sm.dot[pj] * (rj * rj);
+        double *const wn = a.W + (size_t)j * a.n + lo;
+        pj = a.ring > 0 ? (pj + 1 == a.ring ? 0 : pj + 1) : j + 1 - (a.iop ? max(0, j + 2 - a.q) : 0);
+        double *const xn = a.ring > 0 ? slot0 + pj * a.chunk : j + 1 < a.slots ? slot0 + (j + 1) * a.chunk : nullptr;
+        acc = 0.0;
+#pragma unroll 1
+        for (int il = tid; il < len; il += NS * NT) {
+            double u[NS];
+            int off[NS];  // of the states; past the slice: the first one again
+#pragma unroll
+            for (int s = 0; s < NS; ++s) {
+                u[s] = REG ? w[s] : ws[il];
+                off[s] = il + s * NT < len ? s * NT : 0;
+            }
+            const double *p = base + il;
+            const int r4 = min((Kres + 3) & ~3, max(0, a.ring > 0 ? a.slots : a.slots - istart) & ~3);  // past K: c is zero
+            int r = 0;
+#pragma unroll 1
+            for (; r < r4; r += 4, p += 4 * a.chunk) {
+                const double2 c01 = sm.c2[r >> 1], c23 = sm.c2[(r >> 1) + 1];
+#pragma unroll
+                for (int s = 0; s < NS; ++s) {
+                    const double *ps = p + off[s];
+                    u[s] = fma(-c01.y, ps[a.chunk], fma(-c01.x, ps[0], u[s]));
+                    u[s] = fma(-c23.y, ps[3 * a.chunk], fma(-c23.x, ps[2 * a.chunk], u[s]));
+                }
+            }
+#pragma unroll 1
+            for (; r < Kres; ++r, p += a.chunk) {
+#pragma unroll
+                for (int s = 0; s < NS; ++s) u[s] = fma(-c[r], p[off[s]], u[s]);
+            }
+            r = Kres;
+#pragma unroll 2
+            for (; r < K - 1; ++r) {  // positions in L2 (W_j itself follows)
+                const double *g = (istart + r == 0 ? a.v0 + lo : gbase + (size_t)r * a.n) + il;
+#pragma unroll
+                for (int s = 0; s < NS; ++s) u[s] = fma(-c[r], __ldcg(g + off[s]), u[s]);
+            }
+#pragma unroll
+            for (int s = 0; s < NS; ++s) {
+                if (s == 0 || off[s] > 0) {
+                    const int i = il + s * NT;
+                    const double wi = settled(fma(-cj, xs[i], u[s]) * rj);
+                    st_relaxed(wn + i, wi);
+                    acc = fma(wi, wi, acc);
+                    xs[i] = wi;
+                    if (xn) xn[i] = wi;
+                }
             }
         }
+        acc = warp_sum(acc);
+        if (lane == 0) sm.wsum[warp] = acc;
+        x = a.W + (size_t)j * a.n;
         __syncthreads();
-        // w -= sum_k gam_k W_k and ||w||^2
-        acc = 0.0;
-        for (int il = tid; il < len; il += blockDim.x) {
-            double wi = ws[il];
-            for (int k = 0; k < K; ++k) wi = fma(-sm.gam[k], __ldcg(wv(istart + k) + lo + il), wi);
-            __stcg(w + lo + il, wi);
-            acc = fma(wi, wi, acc);
+        if (blockIdx.x == 0) {  // column j of H, while the others' entries travel
+            if (tid < K) {
+                const int k = a.ring > 0 ? tid + a.ring * ((j - tid) / a.ring) : istart + tid;
+                a.H[k + j * a.mp2] = (k == j ? rj : sm.rho[k]) * rj * sm.dot[tid];
+            }
+            if (tid == NT - 1) {
+                a.rho[j] = rj;
+                if (j > 0) a.H[j + (j - 1) * a.mp2] = sn;
+                else {
+                    *a.beta = sn;
+                    *a.avnorm = 0.0;
+                }
+            }
         }
-        if (!reduce1(acc, part(), red, sm, a, epoch)) return;
-        const double sn = sqrt(sm.res[0]);
-        if (!isfinite(sn)) {
-            if (lead) *a.flag = -1;
-            return;
-        }
-        if (sn < a.btol) {
-            if (lead) *a.flag = j + 1;
-            return;
-        }
-        if (tid == 0) sm.rho[j + 1] = 1.0 / sn;
-        if (lead) {
-            a.H[(j + 1) + (size_t)j * mp2] = sn;
-            a.rho[j + 1] = 1.0 / sn;
-        }
-        __syncthreads();
-    }
-    if (a.with_avnorm) {  // ||A v_m|| (src/KryExpvFSP.cu:114-120)
-        const double *x = wv(a.m);
-        double *w = a.W + (size_t)a.m * n;
-        const double rm = sm.rho[a.m];
-        acc = 0.0;
-        for (int il = tid; il < len; il += blockDim.x) {
-            const double wi = rm * term_apply(a, x, lo + il);
-            __stcg(w + lo + il, wi);
-            acc = fma(wi, wi, acc);
-        }
-        if (!reduce1(acc, part(), red, sm, a, epoch)) return;
-        if (lead) {
-            const double av = sqrt(sm.res[0]);
-            *a.avnorm = av;
-            if (!isfinite(av)) *a.flag = -1;
-        }
+        if (tid == 0) sm.rho[j] = rj;
     }
 }
 
@@ -355,10 +496,10 @@ struct PArnoldi {
     int *d_rterm = nullptr;
     int64_t *d_d = nullptr;
     double *d_props = nullptr;  // sparse formats: exported propensities
-    double *d_part = nullptr;
-    unsigned *d_bar = nullptr;  // grid-barrier arrival counter
-    int grid = 0;
-    int64_t chunk = 0;
+    double *d_ex = nullptr;  // two exchange areas: a launch uses one and clears the other
+    int ex_rows = 0;         // rows per area
+    int turn = 0;            // area of the next launch
+    int grid = 0, chunk = 0, slots = 0, ring = 0;
     size_t smem = 0;
 };
 
@@ -373,8 +514,7 @@ void parnoldi_release(PArnoldi *pa, Free release) {
     release(pa->d_rterm);
     release(pa->d_d);
     release(pa->d_props);
-    release(pa->d_part);
-    release(pa->d_bar);
+    release(pa->d_ex);
     delete pa;
 }
 }  // namespace
@@ -514,6 +654,21 @@ cufsp_status build_terms(PArnoldi *pa, cufsp_mat *A, const std::vector<double> &
 }  // namespace
 
 namespace {
+using PKernel = void (*)(const PArgs);
+struct PVariant {
+    PKernel kern;
+    int threads, states, near, far;  // states per CTA, near and far terms it takes
+};
+// the first that fits is used; the last takes everything
+#define CUFSP_PV(NS, TN, TF) {k_arnoldi_persistent<256, NS, TN, TF>, 256, 256 * NS, TN, TF}
+const PVariant kPVariants[] = {CUFSP_PV(1, 4, 2), CUFSP_PV(1, 10, 4), CUFSP_PV(1, 4, 8), CUFSP_PV(2, 4, 2), CUFSP_PV(2, 10, 4),
+                               CUFSP_PV(2, 4, 8), CUFSP_PV(4, 4, 2),  CUFSP_PV(4, 10, 4), CUFSP_PV(4, 4, 8),
+                               {k_arnoldi_persistent<512, 1, 0, 0>, 512, INT32_MAX, kMaxTerms, kMaxTerms}};
+#undef CUFSP_PV
+
+// Dynamic shared memory the pass may use.
+size_t persistent_smem_max() { return (size_t)device_info().max_smem_optin - sizeof(PSmem) - 1024; }
+
 cudaError_t persistent_smem_attribute() {
     constexpr int kMaxDevices = 64;
     static std::mutex mu;
@@ -525,8 +680,10 @@ cudaError_t persistent_smem_attribute() {
     if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
     std::lock_guard<std::mutex> lk(mu);
     if (!done[dev]) {
-        result[dev] = cudaFuncSetAttribute((const void *)k_arnoldi_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           device_info().max_smem_optin - (int)sizeof(PSmem) - 1024);
+        for (const PVariant &v : kPVariants)
+            if (result[dev] == cudaSuccess)
+                result[dev] = cudaFuncSetAttribute((const void *)v.kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)persistent_smem_max());
         done[dev] = true;
     }
     return result[dev];
@@ -551,34 +708,48 @@ cufsp_status parnoldi_run(PArnoldi **ppa, cufsp_mat *A, const std::vector<double
         }();
         // a host thread that shares the GPU with other solves (the batched gradient's workers) takes
         // its share of the SMs, so that the workers' cooperative passes run side by side
-        const int sms = tl_cta_cap > 0 ? std::min(tl_cta_cap, device_info().sm_count) : device_info().sm_count;
-        const int64_t want = std::max<int64_t>(1, std::min<int64_t>(sms, (n + min_states - 1) / min_states));
-        const int64_t chunk = (n + want - 1) / want;
+        const int sms = std::min(device_info().sm_count, 64 * kMaxGridPairs);
+        const int cap = tl_cta_cap > 0 ? std::min(tl_cta_cap, sms) : sms;
+        const int64_t want = std::max<int64_t>(1, std::min<int64_t>(cap, (n + min_states - 1) / min_states));
+        const int64_t chunk = ((n + want - 1) / want + 1) & ~int64_t(1);
         const int64_t grid = (n + chunk - 1) / chunk;
-        const size_t smem = sizeof(double) * ((size_t)chunk + (size_t)std::max(1, m) * grid);
-        if (smem > (size_t)device_info().max_smem_optin - sizeof(PSmem) - 1024)
-            return set_error(CUFSP_ERR_UNSUPPORTED, "persistent Arnoldi: vector slice exceeds shared memory");
+        const size_t row = sizeof(double) * (size_t)chunk, room = persistent_smem_max();
+        if (n > INT32_MAX / 2) return set_error(CUFSP_ERR_UNSUPPORTED, "persistent Arnoldi: too many states");
+        // basis vectors the dots read: W_0..W_{m-1}, or the last q of them
+        const bool window = iop && q < m;
+        const size_t fixed = 2 * row + 2 * kHaloMax * sizeof(double);
+        if (fixed > room) return set_error(CUFSP_ERR_UNSUPPORTED, "persistent Arnoldi: vector slice exceeds shared memory");
+        pa->slots = (int)std::min<size_t>((size_t)(window ? q : m), (room - fixed) / row);
+        pa->ring = window && pa->slots == q ? q : 0;
         // The attribute belongs to the current device: set it once per device, to the most any
         // driver may ask for, so that drivers of different sizes on different host threads never
         // undercut each other.
         CUFSP_CUDA_TRY(persistent_smem_attribute());
-        int per_sm = 0;
-        CUFSP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)k_arnoldi_persistent,
-                                                                     kPThreads, smem));
-        if (per_sm < 1) return set_error(CUFSP_ERR_CUDA, "persistent Arnoldi: kernel does not fit an SM");
+        pa->smem = fixed + row * (size_t)pa->slots;
+        for (const PVariant &v : kPVariants) {
+            int per_sm = 0;
+            CUFSP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)v.kern, v.threads, pa->smem));
+            if (per_sm < 1) return set_error(CUFSP_ERR_CUDA, "persistent Arnoldi: kernel does not fit an SM");
+        }
+        // exchange rows of one launch: K + 1 per iteration, two for the norms at the end
+        int rows = 2;
+        for (int j = 0; j < m; ++j) rows += (iop ? std::min(j + 1, q) : j + 1) + 1;
+        pa->ex_rows = rows;
+        const size_t bytes = sizeof(double) * 2 * (size_t)exchange_doubles(rows, (int)grid);
+        CUFSP_CUDA_TRY(cache_alloc((void **)&pa->d_ex, bytes));
+        CUFSP_CUDA_TRY(cudaMemsetAsync(pa->d_ex, kUnsetByte, bytes, st));
+        pa->chunk = (int)chunk;
         pa->grid = (int)grid;
-        pa->chunk = chunk;
-        pa->smem = smem;
-        CUFSP_CUDA_TRY(cache_alloc((void **)&pa->d_part, sizeof(double) * 2 * (size_t)pa->grid * kKMax));
-        CUFSP_CUDA_TRY(cache_alloc((void **)&pa->d_bar, sizeof(unsigned)));
     }
     PArgs a;
     std::memset(&a, 0, sizeof(a));
-    a.n = n;
+    a.n = (int)n;
     a.chunk = pa->chunk;
+    a.slots = pa->slots;
+    a.ring = pa->ring;
     a.T = tm->T;
     a.coef = tm->d_coef;
-    for (int t = 0; t < tm->T; ++t) a.shift[t] = tm->shift[t];
+    for (int t = 0; t < tm->T; ++t) a.shift[t] = (int)tm->shift[t];
     a.v0 = v;
     a.W = W;
     a.H = H;
@@ -593,14 +764,32 @@ cufsp_status parnoldi_run(PArnoldi **ppa, cufsp_mat *A, const std::vector<double
     a.q = q;
     a.btol = btol;
     a.with_avnorm = with_avnorm ? 1 : 0;
-    a.part = pa->d_part;
-    a.bar = pa->d_bar;
+    const size_t area = (size_t)exchange_doubles(pa->ex_rows, pa->grid);
+    a.ex = pa->d_ex + (size_t)pa->turn * area;
+    a.ex_next = pa->d_ex + (size_t)(1 - pa->turn) * area;
+    a.ex_rows = pa->ex_rows;
     a.err = err;
-    CUFSP_CUDA_TRY(cudaMemsetAsync(pa->d_bar, 0, sizeof(unsigned), st));
-    CUFSP_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int), st));
+    pa->turn = 1 - pa->turn;
+    // near terms read the slice and its halo in shared memory: shifts of up to kHaloMax states
+    int near = 0, far = 0, halo = 0;
+    for (int t = 0; t < a.T; ++t) {
+        const int d = std::abs(a.shift[t]);
+        if (d <= kHaloMax) {
+            if (near < kMaxNear) a.near_t[near] = (short)t;
+            ++near;
+            halo = std::max(halo, d);
+        } else {
+            if (far < kMaxFar) a.far_t[far] = (short)t;
+            ++far;
+        }
+    }
+    a.n_near = near;
+    a.n_far = far;
+    a.halo = (halo + 1) & ~1;
+    const PVariant *var = kPVariants;
+    while (a.chunk > var->states || near > var->near || far > var->far) ++var;
     void *args[] = {&a};
-    CUFSP_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_arnoldi_persistent, dim3(pa->grid), dim3(kPThreads),
-                                               args, pa->smem, st));
+    CUFSP_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)var->kern, dim3(pa->grid), dim3(var->threads), args, pa->smem, st));
     return CUFSP_SUCCESS;
 }
 
