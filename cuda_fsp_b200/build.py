@@ -30,9 +30,9 @@ NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-rdc=true", "-Xcompiler"
 HOST_EXTRA = {"cufsp_expm.cpp": ["-Xcompiler", "-O3"]}
 SOURCES = ["cufsp_common.cu", "cufsp_rtc.cu", "cufsp_kron.cu", "cufsp_kron_plane.cu", "cufsp_kron_march.cu", "cufsp_sparse.cu", "cufsp_mat.cu",
            "cufsp_krylov.cu", "cufsp_expm.cpp", "cufsp_noalloc.cu", "cufsp_stats.cu", "cufsp_solver.cu",
-           "cufsp_vec.cu", "cufsp_bdf.cu", "cufsp_batch.cu", "cufsp_adjoint.cu", "cufsp_adaptive.cu",
+           "cufsp_vec.cu", "cufsp_bdf.cu", "cufsp_bdf_step.cu", "cufsp_batch.cu", "cufsp_adjoint.cu", "cufsp_adaptive.cu",
            "cufsp_arnoldi.cu"]
-HEADERS = ["cufsp_internal.h", "cufsp_reduce.cuh", "cufsp_grid.cuh", "cufsp_march.h", "cufsp_vec.h", "cufsp_plane.cuh", "cufsp_batch.cuh",
+HEADERS = ["cufsp_internal.h", "cufsp_reduce.cuh", "cufsp_grid.cuh", "cufsp_slice.cuh", "cufsp_bdf_step.h", "cufsp_march.h", "cufsp_vec.h", "cufsp_plane.cuh", "cufsp_batch.cuh",
            "cufsp_sparse_rtc.cuh", "cufsp_kron_rtc.cuh"]
 # Kernel sources compiled at run time by NVRTC are embedded in the library as string literals.
 RTC_SOURCES = {"cufsp_plane.cuh": "cufsp_plane_src.inc", "cufsp_batch.cuh": "cufsp_batch_src.inc",

@@ -21,7 +21,8 @@
 //    in registers for the whole launch, and sources inside the slice come from shared memory.
 //  * the CTA's slices of as many basis vectors as fit live in shared memory (all 30 of them up to 148 x
 //    ~890 = 131K states); the dots and the update read them there and the rest from L2.
-// Measured, one pass of m = 30 (events around the launch): @PASS@
+// Measured, a Krylov step of m = 30 (pass, host step control and combination): 32,768 states 0.35 ms with
+// two barriers per iteration, 0.20 ms so; 134,088 states 0.50 and 0.28 ms.
 // Waits are bounded; on expiry the kernel sets an error word, every CTA leaves, and the host reports
 // CUFSP_ERR_CUDA.  The launch is cooperative, so all CTAs are co-resident.
 #include <algorithm>
@@ -34,18 +35,18 @@
 
 #include "cufsp_internal.h"
 #include "cufsp_grid.cuh"
+#include "cufsp_slice.cuh"
 
 namespace cufsp {
 
 namespace {
 
 constexpr int kMaxTerms = 64;
-constexpr int kHaloMax = 64;   // largest |shift| of a term whose sources are read from shared memory
-constexpr int kMaxNear = 10, kMaxFar = 8;
 constexpr int kPThreadsMax = 512;
 constexpr int kPWarpsMax = kPThreadsMax / 32;
 
 struct PArgs {
+    SliceTerms terms;           // register variants
     int n;
     int chunk;                  // states per CTA, even (the last CTA may have fewer)
     int slots;                  // basis vectors whose slices live in shared memory
@@ -53,9 +54,6 @@ struct PArgs {
     int T;
     const double *coef;         // [T][n]
     int shift[kMaxTerms];       // source index i - shift[t] (clamped)
-    // register variants: the terms with |shift| <= halo, and the others (term, -1: none)
-    int n_near, n_far, halo;
-    short near_t[kMaxNear], far_t[kMaxFar];
     const double *v0;           // W_0 (the caller's vector)
     double *W;                  // W_1 .. W_{m+1}
     double *H, *rho, *gam, *beta, *avnorm;
@@ -78,9 +76,8 @@ struct PSmem {
     double sn, rj;                           // ||W_j||, 1 / ||W_j||
 };
 
-// NT threads.  TN > 0: at most NS states per thread, TN near and TF far terms, coefficients in registers;
-// the near terms' sources come from the slice in shared memory, extended on both sides by a halo of the
-// neighbours' entries, the far terms' from L2, all loads of a thread in flight together.  TN = 0: any.
+// NT threads.  TN > 0: at most NS states per thread, TN near and TF far terms (cufsp_slice.cuh), their
+// coefficients in registers.  TN = 0: any.
 // 8 warps with up to 4 states per thread rather than 16 or 32 with fewer: at these sizes the instructions
 // that every warp spends on addresses, reductions and waits, not the data, fill an iteration between two
 // waits, and a thread of 8 warps has 255 registers, so that nothing spills (a spill goes to L2: shared
@@ -96,8 +93,8 @@ __global__ void __launch_bounds__(NT, 1) k_arnoldi_persistent(const __grid_const
     const int len = min(a.chunk, a.n - lo);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool lead = blockIdx.x == 0 && tid == 0;
-    double *const xs = ws + a.chunk + a.halo;
-    double *const slot0 = xs + a.chunk + a.halo;
+    double *const xs = ws + a.chunk + a.terms.halo;
+    double *const slot0 = xs + a.chunk + a.terms.halo;
     double *const c = reinterpret_cast<double *>(sm.c2);
     const int pitch = exchange_pitch((int)gridDim.x);
 
@@ -109,7 +106,7 @@ __global__ void __launch_bounds__(NT, 1) k_arnoldi_persistent(const __grid_const
         for (int i = tid; i < a.mp2 * (a.mp2 + 2); i += NT) a.H[i] = 0.0;  // H, rho and gam are contiguous
     }
 #pragma unroll 1
-    for (int il = tid; il < (a.slots + 2) * a.chunk + 2 * a.halo; il += NT) ws[il] = 0.0;
+    for (int il = tid; il < (a.slots + 2) * a.chunk + 2 * a.terms.halo; il += NT) ws[il] = 0.0;
     if (tid < CUFSP_MAX_KRYLOV + 4) c[tid] = 0.0;  // positions a loop rounded up to four may read
     __syncthreads();
     double cn[NS][REG ? TN : 1], cfar[NS][REG ? TF : 1];
@@ -119,9 +116,9 @@ __global__ void __launch_bounds__(NT, 1) k_arnoldi_persistent(const __grid_const
             const int il = tid + s * NT;
             const double *cp = a.coef + lo + il;
 #pragma unroll
-            for (int t = 0; t < TN; ++t) cn[s][t] = t < a.n_near && il < len ? __ldcg(cp + (size_t)a.near_t[t] * a.n) : 0.0;
+            for (int t = 0; t < TN; ++t) cn[s][t] = t < a.terms.n_near && il < len ? __ldcg(cp + (size_t)a.terms.near_t[t] * a.n) : 0.0;
 #pragma unroll
-            for (int t = 0; t < TF; ++t) cfar[s][t] = t < a.n_far && il < len ? __ldcg(cp + (size_t)a.far_t[t] * a.n) : 0.0;
+            for (int t = 0; t < TF; ++t) cfar[s][t] = t < a.terms.n_far && il < len ? __ldcg(cp + (size_t)a.terms.far_t[t] * a.n) : 0.0;
         }
     }
     double acc = 0.0;
@@ -154,76 +151,26 @@ __global__ void __launch_bounds__(NT, 1) k_arnoldi_persistent(const __grid_const
         double *const mine = a.ex + (size_t)row * pitch + blockIdx.x;
         double w[NS];
         double aw2 = 0.0;
-        Patience wait;
         bool bad = false;
         if (warp == NW - 1 && j > 0) {  // row 0: ||W_j||^2, on its way while A W_j is formed
             const double v = warp_sum(lane < NW ? sm.wsum[lane] : 0.0);
             if (lane == 0) st_relaxed(mine, settled(v));
         }
-        // entry rel of the slice from L2 (unset until its owner has stored it)
-        auto far = [&](int rel) -> double { return ld_relaxed(x + min(max(lo + rel, 0), a.n - 1)); };
         if (!last || a.with_avnorm) {
             if constexpr (REG) {
                 double v[NS][TF];
-#pragma unroll
-                for (int s = 0; s < NS; ++s)
-#pragma unroll
-                    for (int t = 0; t < TF; ++t) {
-                        v[s][t] = 0.0;
-                        if (t < a.n_far && s * NT < len) v[s][t] = far(tid + s * NT - a.shift[a.far_t[t]]);
-                    }
-                if (tid < 2 * a.halo) {
-                    const int rel = tid < a.halo ? tid - a.halo : len + tid - a.halo;
-                    double h = far(rel);
-                    while (j > 0 && is_unset(h)) {
-                        if (wait.give_up(a.err)) {
-                            bad = true;
-                            break;
-                        }
-                        h = far(rel);
-                    }
-                    xs[rel] = h;
-                }
+                bad = !gather_begin<NT, NS, TF>(a.terms, x, lo, len, j > 0, xs, v, a.err);
                 __syncthreads();
-#pragma unroll
-                for (int s = 0; s < NS; ++s) w[s] = 0.0;
-#pragma unroll
-                for (int t = 0; t < TN; ++t) {
-                    if (t >= a.n_near) break;
-                    const double *p = xs + tid - a.shift[a.near_t[t]];
-#pragma unroll
-                    for (int s = 0; s < NS; ++s)
-                        if (tid + s * NT < len) w[s] = fma(cn[s][t], p[s * NT], w[s]);
-                }
-                if (j > 0) {
-                    for (;;) {
-                        bool miss = false;
-#pragma unroll
-                        for (int s = 0; s < NS; ++s)
-#pragma unroll
-                            for (int t = 0; t < TF; ++t)
-                                if (is_unset(v[s][t])) {
-                                    miss = true;
-                                    v[s][t] = far(tid + s * NT - a.shift[a.far_t[t]]);
-                                }
-                        if (!miss) break;
-                        if (wait.give_up(a.err)) {
-                            bad = true;
-                            break;
-                        }
-                    }
-                }
+                if (!gather_end<NT, NS, TN, TF>(a.terms, x, lo, len, j > 0, xs, cn, cfar, v, w, a.err)) bad = true;
 #pragma unroll
                 for (int s = 0; s < NS; ++s) {
-#pragma unroll
-                    for (int t = 0; t < TF; ++t) w[s] = fma(cfar[s][t], v[s][t], w[s]);
                     if (tid + s * NT < len) ws[tid + s * NT] = w[s];
-                    else w[s] = 0.0;
                     aw2 = fma(w[s], w[s], aw2);
                 }
             } else {
 #pragma unroll 1
                 for (int il = tid; il < len; il += NT) {
+                    Patience wait;
                     double sum;
                     bool miss;
                     do {
@@ -234,7 +181,7 @@ __global__ void __launch_bounds__(NT, 1) k_arnoldi_persistent(const __grid_const
                             const int rel = il - a.shift[t];
                             double v;
                             if ((unsigned)rel < (unsigned)len) v = xs[rel];
-                            else v = far(rel);
+                            else v = far_entry(x, lo, rel, a.n);
                             miss = miss || is_unset(v);
                             sum = fma(__ldg(a.coef + (size_t)t * a.n + lo + il), v, sum);
                         }
@@ -251,54 +198,12 @@ __global__ void __launch_bounds__(NT, 1) k_arnoldi_persistent(const __grid_const
             if (lane == 0) sm.asum[warp] = aw2;
         }
         if (__syncthreads_or(bad)) return;
-        // dots over the slice: a warp takes four positions and one part of the slice, so that each entry
-        // of A W_j is read once for four products
-        const int lnb = K > 32 ? 4 : K > 16 ? 3 : K > 8 ? 2 : K > 4 ? 1 : 0, nb = 1 << lnb;
-        const int nsl = NW >> lnb;  // parts (0: more groups of four than warps)
-#pragma unroll 1
-        for (int r0 = (warp & (nb - 1)) * 4, part = warp; r0 < K; r0 += 4 * NW, part += NW) {
-            const int half = a.chunk >> 1, per = nsl > 1 ? (half + nsl - 1) >> (LNW - lnb) : half;
-            const int b0 = nsl > 1 ? (warp >> lnb) * per : 0, b1 = min(half, b0 + per);
-            const int q1 = min(r0 + 1, K - 1), q2 = min(r0 + 2, K - 1), q3 = min(r0 + 3, K - 1);
-            double d0 = 0.0, d1 = 0.0, d2 = 0.0, d3 = 0.0;
-            if (q3 < Kres) {
-                const double2 *p0 = reinterpret_cast<const double2 *>(base + r0 * a.chunk);
-                const double2 *p1 = reinterpret_cast<const double2 *>(base + q1 * a.chunk);
-                const double2 *p2 = reinterpret_cast<const double2 *>(base + q2 * a.chunk);
-                const double2 *p3 = reinterpret_cast<const double2 *>(base + q3 * a.chunk);
-                const double2 *pw = reinterpret_cast<const double2 *>(ws);
-#pragma unroll 2
-                for (int b = b0 + lane; b < b1; b += 32) {
-                    const double2 u = pw[b], u0 = p0[b], u1 = p1[b], u2 = p2[b], u3 = p3[b];
-                    d0 = fma(u0.y, u.y, fma(u0.x, u.x, d0));
-                    d1 = fma(u1.y, u.y, fma(u1.x, u.x, d1));
-                    d2 = fma(u2.y, u.y, fma(u2.x, u.x, d2));
-                    d3 = fma(u3.y, u.y, fma(u3.x, u.x, d3));
-                }
-            } else {
-                const double *p0 = istart + r0 == 0 ? a.v0 + lo : gbase + (size_t)r0 * a.n;
-                const double *p1 = gbase + (size_t)q1 * a.n, *p2 = gbase + (size_t)q2 * a.n, *p3 = gbase + (size_t)q3 * a.n;
-                if (istart + q1 == 0) p1 = p2 = p3 = p0;  // K = 1
-#pragma unroll 4
-                for (int il = 2 * b0 + lane; il < min(len, 2 * b1); il += 32) {
-                    const double u = ws[il];
-                    d0 = fma(__ldcg(p0 + il), u, d0);
-                    d1 = fma(__ldcg(p1 + il), u, d1);
-                    d2 = fma(__ldcg(p2 + il), u, d2);
-                    d3 = fma(__ldcg(p3 + il), u, d3);
-                }
-            }
-            d0 = warp_sum4(d0, d1, d2, d3);
-            if ((lane & 7) == 0) sm.part[part][lane >> 3] = d0;
-        }
+        slice_dots<LNW>(ws, a.chunk, len, K, Kres, base, istart == 0 ? a.v0 + lo : gbase, gbase, a.n, sm.part);
         __syncthreads();
         // publish the other rows: the dots, or ||A W_m||^2
         if (j == 0) __threadfence();  // the cleared basis is visible before any CTA passes this exchange
         if (tid < K) {
-            double v = sm.part[tid >> 2][tid & 3];
-#pragma unroll 4
-            for (int u = 1; u < nsl; ++u) v += sm.part[(u << lnb) + (tid >> 2)][tid & 3];
-            st_relaxed(mine + (size_t)(1 + tid) * pitch, settled(v));
+            st_relaxed(mine + (size_t)(1 + tid) * pitch, settled(dots_sum<LNW>(sm.part, K, tid)));
         }
         if (warp == NW - 1 && (last || j == 0)) {
             const double v = warp_sum(lane < NW ? (last ? sm.asum : sm.wsum)[lane] : 0.0);
@@ -770,24 +675,10 @@ cufsp_status parnoldi_run(PArnoldi **ppa, cufsp_mat *A, const std::vector<double
     a.ex_rows = pa->ex_rows;
     a.err = err;
     pa->turn = 1 - pa->turn;
-    // near terms read the slice and its halo in shared memory: shifts of up to kHaloMax states
-    int near = 0, far = 0, halo = 0;
-    for (int t = 0; t < a.T; ++t) {
-        const int d = std::abs(a.shift[t]);
-        if (d <= kHaloMax) {
-            if (near < kMaxNear) a.near_t[near] = (short)t;
-            ++near;
-            halo = std::max(halo, d);
-        } else {
-            if (far < kMaxFar) a.far_t[far] = (short)t;
-            ++far;
-        }
-    }
-    a.n_near = near;
-    a.n_far = far;
-    a.halo = (halo + 1) & ~1;
+    a.terms.n = (int)n;
+    split_terms(a.T, a.shift, a.terms);
     const PVariant *var = kPVariants;
-    while (a.chunk > var->states || near > var->near || far > var->far) ++var;
+    while (a.chunk > var->states || a.terms.n_near > var->near || a.terms.n_far > var->far) ++var;
     void *args[] = {&a};
     CUFSP_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)var->kern, dim3(pa->grid), dim3(var->threads), args, pa->smem, st));
     return CUFSP_SUCCESS;

@@ -26,6 +26,7 @@
 #include <cstring>
 #include <vector>
 
+#include "cufsp_bdf_step.h"
 #include "cufsp_internal.h"
 #include "cufsp_reduce.cuh"
 #include "cufsp_vec.h"
@@ -34,8 +35,9 @@ using namespace cufsp;
 
 namespace {
 
-constexpr int kMaxOrder = 5;
+constexpr int kMaxOrder = kBdfOrder;
 constexpr int kNHist = kMaxOrder + 3;
+static_assert(kNHist == kBdfHist, "difference history");
 constexpr int kMaxL = 60;
 
 // device scalar block (doubles)
@@ -173,6 +175,8 @@ struct cufsp_bdf_s {
     double t = 0.0, h = 0.0;
     int order = 1, n_equal = 0;
     cufsp_bdf_stats st{};
+    BdfStepper *stepper = nullptr;  // step attempts as one launch each; null: the launch sequence
+    bool stepper_asked = false;
 
     double *vec(int j) const { return V + (int64_t)j * ld; }
 };
@@ -374,11 +378,50 @@ cufsp_status gmres(cufsp_bdf *B, double t, double c, cudaStream_t st, int *conv)
     return vec_lincomb(n, J, vp, y, B->d, false, B->w, B->d_scal + kErr, B->rs, st);
 }
 
+// One step attempt as a single launch (cufsp_bdf_step.cu): *conv, *err and, when the step is accepted
+// (err <= 1), the updated history with the norms of D_k and D_{k+2}.
+cufsp_status attempt(cufsp_bdf *B, double t_new, double c, cudaStream_t st, int *conv, double *err, double *em,
+                     double *ep) {
+    BDF_TRY(mat_coefs(B->A, t_new, B->fixed ? B->coefs.data() : nullptr, B->cbuf));
+    BdfStepIn in;
+    for (int j = 0; j < kNHist; ++j) in.D[j] = B->D[j];
+    in.w = B->w;
+    in.k = B->order;
+    for (int j = 0; j <= kMaxOrder; ++j) in.g[j] = B->gam[j];
+    in.inv_alpha = 1.0 / B->gam[B->order];
+    in.c = c;
+    in.econst = B->econst[B->order];
+    in.atol = B->atol;
+    in.rtol = B->rtol;
+    in.sqrt_n = std::sqrt((double)B->n);
+    in.eps_lin = B->eps_lin;
+    in.coefs = B->cbuf.data();
+    in.h_out = B->h_scal;
+    in.h_seq = B->h_seq;
+    in.seq = &B->seq;
+    static_assert(kBdfOutWords <= kNScal, "report block");
+    BdfStepOut out;
+    BDF_TRY(bdf_stepper_run(B->stepper, in, out, st));
+    B->st.n_matvec += 1 + out.iters;
+    B->st.n_lin_iters += out.iters;
+    if (out.status == kBdfRhsNonfinite) return set_error(CUFSP_ERR_NONFINITE, "cufsp_bdf: right-hand side is not finite");
+    if (out.status == kBdfBasisNonfinite) return set_error(CUFSP_ERR_NONFINITE, "cufsp_bdf: Krylov vector is not finite");
+    *conv = out.status != kBdfNotConverged;
+    *err = out.err;
+    *em = out.em;
+    *ep = out.ep;
+    return CUFSP_SUCCESS;
+}
+
 // One attempt sequence ending in an accepted step toward t_out (never past it).
 cufsp_status step(cufsp_bdf *B, double t_out, cudaStream_t st) {
     const int64_t n = B->n;
     const double eps = 2.220446049250313e-16;
     const double hmax = B->h_max > 0.0 ? B->h_max : INFINITY;
+    if (!B->stepper_asked) {
+        B->stepper_asked = true;
+        B->stepper = bdf_stepper_create(B->A, B->maxl, st);
+    }
     for (;;) {
         if (B->h > hmax) {
             BDF_TRY(change_D(B, B->order, hmax / B->h, st));
@@ -398,12 +441,23 @@ cufsp_status step(cufsp_bdf *B, double t_out, cudaStream_t st) {
         const int k = B->order;
         const double t_new = landing ? t_out : B->t + B->h;
         const double alpha = B->gam[k], c = B->h / alpha;
-        k_bdf_predict<<<grid_of(n), 256, 0, st>>>(hist(B, k), B->ypred, B->vec(0), B->gam[1], B->gam[2], B->gam[3],
-                                                  B->gam[4], B->gam[5], 1.0 / alpha);
-        CUFSP_CUDA_TRY(cudaGetLastError());
-        BDF_TRY(apply(B, t_new, c, B->ypred, true, B->vec(0), st));
         int conv = 0;
-        BDF_TRY(gmres(B, t_new, c, st, &conv));
+        double err = 0.0, em_norm = 0.0, ep_norm = 0.0;
+        bool updated = false;  // the history has taken the step
+        if (B->stepper) {
+            BDF_TRY(attempt(B, t_new, c, st, &conv, &err, &em_norm, &ep_norm));
+            updated = conv && err <= 1.0;
+        } else {
+            k_bdf_predict<<<grid_of(n), 256, 0, st>>>(hist(B, k), B->ypred, B->vec(0), B->gam[1], B->gam[2], B->gam[3],
+                                                      B->gam[4], B->gam[5], 1.0 / alpha);
+            CUFSP_CUDA_TRY(cudaGetLastError());
+            BDF_TRY(apply(B, t_new, c, B->ypred, true, B->vec(0), st));
+            BDF_TRY(gmres(B, t_new, c, st, &conv));
+            if (conv) {
+                BDF_TRY(fetch(B, kErr, 1, st));
+                err = B->econst[k] * B->h_scal[kErr];
+            }
+        }
         if (!conv) {
             B->st.n_lin_fail++;
             BDF_TRY(change_D(B, k, 0.5, st));
@@ -411,8 +465,6 @@ cufsp_status step(cufsp_bdf *B, double t_out, cudaStream_t st) {
             B->n_equal = 0;
             continue;
         }
-        BDF_TRY(fetch(B, kErr, 1, st));
-        const double err = B->econst[k] * B->h_scal[kErr];
         if (!std::isfinite(err)) return set_error(CUFSP_ERR_NONFINITE, "cufsp_bdf: local error estimate is not finite");
         if (err > 1.0) {
             const double rho = std::max(0.2, 0.9 * std::pow(err, -1.0 / (k + 1)));
@@ -422,18 +474,24 @@ cufsp_status step(cufsp_bdf *B, double t_out, cudaStream_t st) {
             B->st.n_reject++;
             continue;
         }
-        k_bdf_accept<<<stream_grid(n, 4, std::min(device_info().sm_count * 4, B->rs.max_ctas)), kRedThreads, 0, st>>>(
-            hist(B, k), B->d, B->w, B->atol, B->rtol, std::sqrt((double)n), B->rs.partials, B->rs.counter,
-            B->d_scal + kEm);
-        CUFSP_CUDA_TRY(cudaGetLastError());
+        if (!updated) {
+            k_bdf_accept<<<stream_grid(n, 4, std::min(device_info().sm_count * 4, B->rs.max_ctas)), kRedThreads, 0, st>>>(
+                hist(B, k), B->d, B->w, B->atol, B->rtol, std::sqrt((double)n), B->rs.partials, B->rs.counter,
+                B->d_scal + kEm);
+            CUFSP_CUDA_TRY(cudaGetLastError());
+        }
         B->t = t_new;
         B->st.n_steps++;
         B->n_equal++;
         B->st.last_err = err;
         if (B->n_equal >= k + 1) {
-            BDF_TRY(fetch(B, kEm, 2, st));
-            const double em = k > 1 ? B->econst[k - 1] * B->h_scal[kEm] : INFINITY;
-            const double ep = k < kMaxOrder ? B->econst[k + 1] * B->h_scal[kEp] : INFINITY;
+            if (!updated) {
+                BDF_TRY(fetch(B, kEm, 2, st));
+                em_norm = B->h_scal[kEm];
+                ep_norm = B->h_scal[kEp];
+            }
+            const double em = k > 1 ? B->econst[k - 1] * em_norm : INFINITY;
+            const double ep = k < kMaxOrder ? B->econst[k + 1] * ep_norm : INFINITY;
             const double fm = std::pow(em, -1.0 / k), f0 = std::pow(err, -1.0 / (k + 1)),
                          fp = std::pow(ep, -1.0 / (k + 2));
             int delta = 0;
@@ -457,6 +515,8 @@ cufsp_status step(cufsp_bdf *B, double t_out, cudaStream_t st) {
 }
 
 void release(cufsp_bdf *B) {
+    bdf_stepper_destroy(B->stepper);
+    B->stepper = nullptr;
     if (B->store) cudaFree(B->store);
     if (B->d_scal) cudaFree(B->d_scal);
     if (B->h_scal) cudaFreeHost(B->h_scal);
