@@ -42,8 +42,12 @@ const char *kBatchSource =
 struct BatchKernel {
     cudaLibrary_t lib = nullptr;
     cudaKernel_t k = nullptr;
-    int smem = 0;
+    int smem = 0;  // the solver's state; the instance tables may follow it
 };
+
+// Instance tables (the rates times the shifted factors) of up to this size go to shared memory, behind the
+// solver's 80 KB: two CTAs per SM still fit.  Larger ones are read through L1 from the workspace.
+constexpr int kTabSmemMax = 32 * 1024;
 
 std::mutex g_batch_mu;
 std::map<std::string, std::shared_ptr<BatchKernel>> g_batch_cache;
@@ -104,7 +108,8 @@ std::shared_ptr<BatchKernel> load_kernel_locked(const std::string &src, const st
     if (e == cudaSuccess) e = cudaLibraryGetGlobal(&dptr, &bytes, bk->lib, "cufsp_batch_smem_bytes");
     if (e == cudaSuccess) e = cudaMemcpy(&bk->smem, dptr, sizeof(int), cudaMemcpyDeviceToHost);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute((const void *)bk->k, cudaFuncAttributeMaxDynamicSharedMemorySize, bk->smem);
+        e = cudaFuncSetAttribute((const void *)bk->k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 bk->smem + kTabSmemMax);
     if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)bk->k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -206,6 +211,8 @@ struct cufsp_batch_s {
     std::vector<int64_t> offsets;          // packed layout, n_inst + 1
     std::vector<int> order;                // largest first
     int64_t n_max = 0;
+    int stride_max = 0;                    // largest tab_stride
+    int tab_smem = 0;                      // bytes of the instance tables in shared memory (0: in the workspace)
     std::string pattern;                   // NVRTC prefix without the launch shape
     CufspBatchInst *d_inst = nullptr;
     int *d_order = nullptr, *d_order_sample = nullptr;
@@ -251,7 +258,7 @@ int clusters_for(cufsp_batch *B, const BatchKernel &k, int cluster, int threads)
     attr[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3(cluster * 64);
     cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = k.smem;
+    cfg.dynamicSmemBytes = k.smem + B->tab_smem;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
@@ -262,8 +269,17 @@ int clusters_for(cufsp_batch *B, const BatchKernel &k, int cluster, int threads)
     return std::min(n, B->n_inst);
 }
 
+// Basis vectors start on 16-byte boundaries: their stride in doubles.
+long long ld_max(const cufsp_batch *B) { return (B->n_max + 1) & ~(int64_t)1; }
+
+// Doubles of one cluster's workspace: m + 1 basis vectors, and the tables of up to 16 CTAs.
+long long work_stride(const cufsp_batch *B) {
+    const long long tabs = B->tab_smem ? 0 : 16LL * (B->nr + 1) * B->stride_max;
+    return (B->m + 1) * ld_max(B) + ((tabs + 1) & ~1LL);
+}
+
 cufsp_status ensure_work(cufsp_batch *B, int n_clusters) {
-    const size_t need = (size_t)n_clusters * (size_t)(B->m + 1) * (size_t)B->n_max;
+    const size_t need = (size_t)n_clusters * (size_t)work_stride(B);
     if (need <= B->work_doubles) return CUFSP_SUCCESS;
     if (B->d_work) cudaFree(B->d_work);
     B->d_work = nullptr;
@@ -282,7 +298,9 @@ cufsp_status launch(cufsp_batch *B, const BatchKernel &k, int cluster, int threa
     a.tables = B->d_tables;
     a.p = p;
     a.work = B->d_work;
-    a.work_stride = (long long)(B->m + 1) * B->n_max;
+    a.work_stride = work_stride(B);
+    a.ld_max = (int)ld_max(B);
+    a.stride_max = B->stride_max;
     a.counter = B->d_counter;
     a.stats = B->d_stats;
     a.n_inst = n_inst;
@@ -300,7 +318,7 @@ cufsp_status launch(cufsp_batch *B, const BatchKernel &k, int cluster, int threa
     attr[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3((unsigned)(cluster * n_clusters));
     cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = k.smem;
+    cfg.dynamicSmemBytes = k.smem + B->tab_smem;
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
@@ -313,7 +331,7 @@ std::string describe_shape(const cufsp_batch *B) {
     std::ostringstream d;
     d << "batched Krylov (NVRTC, sm_100a, one persistent launch): " << B->n_inst << " instances, m=" << B->m
       << (B->iop ? " IOP" : "") << ", " << B->n_clusters << " clusters x " << B->cluster << " CTAs x " << B->threads
-      << " threads (" << B->minb << " CTA/SM bound), smem " << B->kern->smem << " B/CTA";
+      << " threads (" << B->minb << " CTA/SM bound), smem " << B->kern->smem + B->tab_smem << " B/CTA";
     if (B->tune_s > 0.0)
         d << "; autotuner " << std::fixed << std::setprecision(1) << B->tune_s << " s on " << B->n_sample
           << " instances (compiles " << B->tune_compile_s << " s)";
@@ -497,6 +515,7 @@ extern "C" cufsp_status cufsp_batch_create(const cufsp_batch_desc *d, int m, dou
         I.tab = tab_off_inst[i];
         tab_off_inst[i + 1] = tab_off_inst[i] + (int64_t)nr * tsz;
         B->n_max = std::max<int64_t>(B->n_max, n);
+        B->stride_max = std::max(B->stride_max, I.tab_stride);
     }
     for (size_t k = 0; k < B->kinds.size(); ++k) B->kinds[k] = is_one[k] ? 0 : (is_id[k] ? 1 : 2);
     B->order.resize(ni);
@@ -511,7 +530,10 @@ extern "C" cufsp_status cufsp_batch_create(const cufsp_batch_desc *d, int m, dou
     for (int i = 0; i < ni && (int)sample.size() < kSampleMax; i += stride_s) sample.push_back(B->order[i]);
     B->n_sample = (int)sample.size();
 
+    const int64_t tab_bytes = (int64_t)sizeof(double) * (nr + 1) * B->stride_max;
+    B->tab_smem = tab_bytes <= kTabSmemMax ? (int)tab_bytes : 0;
     std::ostringstream s;
+    s << "#define CUFSP_BATCH_TABSMEM " << (B->tab_smem ? 1 : 0) << "\n";
     s << "#define CUFSP_BATCH_NS " << ns << "\n#define CUFSP_BATCH_NR " << nr << "\n#define CUFSP_BATCH_M " << m
       << "\n#define CUFSP_BATCH_IOP " << B->iop << "\n#define CUFSP_BATCH_QIOP " << q_iop << "\nnamespace cufsp_batch {\n";
     emit_fn2(s, "nu", B->nu, ns);

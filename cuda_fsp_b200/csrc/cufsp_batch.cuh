@@ -61,10 +61,11 @@ struct CufspBatchArgs {
     const double *tables;    // packed factor tables
     double *p;               // packed state vectors (in: p(0), out: p(t_final))
     double *work;            // per-cluster basis workspace, work_stride doubles each
-    long long work_stride;   // >= (M + 1) * max n
+    long long work_stride;   // >= (M + 1) ld_max, and the CTAs' tables where they are not in shared memory; even
     unsigned *counter;       // work counter (zero before the launch)
     CufspBatchStat *stats;   // per instance
     int n_inst;
+    int ld_max, stride_max;  // longest basis vector (even), largest tab_stride
     int max_steps, max_reject;
     double t_final, tol, anorm;
 };
@@ -99,9 +100,9 @@ struct Shared {
     double warp_part[WARPS][KR];
     double tot[KR];             // cluster totals
     double H[MP2 * MP2];        // Hessenberg matrix (column-major), identical in every CTA
-    double rho[MP2], gam[MP2];
+    double rho[MP2], gam[MP2 + 8];
     double pade[8][MP2 * MP2];  // exponential workspace
-    double coefc[MP2];          // combination coefficients
+    double coefc[MP2 + 8];          // combination coefficients
     int piv[MP2];
     CufspBatchInst in;          // current instance
     int inst_idx;
@@ -112,95 +113,162 @@ struct Shared {
 // Cluster-wide sum of one value per thread: every CTA ends with the total in s.tot[0].
 __device__ __forceinline__ void cluster_sum1(cg::cluster_group &cl, Shared &s, double v, int &buf);
 
-// Constants of the current instance, copied into registers for the generator action.
-struct Regs {
-    double coef[NR];
-    int delta[NR];
-    int dims[NS];
-    CufspBatchDiv div[NS];
-    int tab_off[NS];
-    int tab_stride;
+// ---- generator action from per-instance tables ----------------------------------------------------
+// At the start of an instance every CTA writes its rates into tables (shared memory when they fit beside
+// the solver's state, else the cluster's workspace): gain[r][s][x_s], the factor of reaction r at the
+// source state x - nu_r, 0 where that leaves the box, with the rate in the first species' factor; and
+// loss[s][x_s], the summed outflow of the reactions whose propensity depends on species s alone.  A state
+// then needs no bounds tests, conversions or factor products of its own: 5 + 16 table reads for the
+// 12-reaction gene network instead of about 300 instructions.
+__device__ constexpr bool used(int r, int sp) { return kind(r, sp) != 0 || nu(r, sp) != 0; }
+__device__ constexpr int first_used(int r) {
+    for (int sp = 0; sp < NS; ++sp)
+        if (used(r, sp)) return sp;
+    return -1;
+}
+__device__ constexpr bool same_nu(int a, int b) {
+    for (int sp = 0; sp < NS; ++sp)
+        if (nu(a, sp) != nu(b, sp)) return false;
+    return true;
+}
+__device__ constexpr int leader(int r) {  // first reaction with r's net change: they share the source entry
+    for (int a = 0; a < r; ++a)
+        if (same_nu(a, r)) return a;
+    return r;
+}
+__device__ constexpr int own_species(int r) {  // the species r's propensity depends on; -1 none, -2 several
+    int at = -1;
+    for (int sp = 0; sp < NS; ++sp)
+        if (kind(r, sp) != 0) at = at == -1 ? sp : -2;
+    return at;
+}
+
+struct Tables {
+    const double *gain;  // [NR][tab_stride]
+    const double *loss;  // [tab_stride]
 };
 
-__device__ __forceinline__ void load_regs(const CufspBatchInst &in, Regs &g) {
-#pragma unroll
-    for (int r = 0; r < NR; ++r) {
-        g.coef[r] = in.coef[r];
-        g.delta[r] = in.delta[r];
-    }
-#pragma unroll
-    for (int sp = 0; sp < NS; ++sp) {
-        g.dims[sp] = in.dims[sp];
-        g.div[sp] = in.div[sp];
-        g.tab_off[sp] = in.tab_off[sp];
-    }
-    g.tab_stride = in.tab_stride;
-}
-
-// Factor f_{r,s}(x) of the current instance.
 template <int R, int SP>
-__device__ __forceinline__ double factor(const Regs &g, const double *__restrict__ tab, int x) {
-    if constexpr (kind(R, SP) == 0) return 1.0;
-    else if constexpr (kind(R, SP) == 1) return (double)x;
-    else return __ldg(tab + R * g.tab_stride + g.tab_off[SP] + x);
-}
-
-template <int R, int SP>
-__device__ __forceinline__ void src_factor(const Regs &g, const double *__restrict__ tab, const int (&x)[NS], double &f,
-                                           bool &ok) {
+__device__ __forceinline__ double gain_factor(const CufspBatchInst &in, const Tables &t, const int (&x)[NS], double f) {
     if constexpr (SP < NS) {
-        const int xs = x[SP] - nu(R, SP);
-        if constexpr (nu(R, SP) > 0) ok = ok && xs >= 0;
-        if constexpr (nu(R, SP) < 0) ok = ok && xs < g.dims[SP];
-        if constexpr (kind(R, SP) != 0) f *= factor<R, SP>(g, tab, min(max(xs, 0), g.dims[SP] - 1));
-        src_factor<R, SP + 1>(g, tab, x, f, ok);
+        if constexpr (used(R, SP)) {
+            const double g = t.gain[R * in.tab_stride + in.tab_off[SP] + x[SP]];
+            f = SP == first_used(R) ? g : f * g;
+        }
+        return gain_factor<R, SP + 1>(in, t, x, f);
     }
+    return f;
 }
 
-template <int R, int SP>
-__device__ __forceinline__ void own_factor(const Regs &g, const double *__restrict__ tab, const int (&x)[NS], double &f) {
-    if constexpr (SP < NS) {
-        if constexpr (kind(R, SP) != 0) f *= factor<R, SP>(g, tab, x[SP]);
-        own_factor<R, SP + 1>(g, tab, x, f);
-    }
-}
-
-// (A v)[i] for one state: sum_r c_r (a_r(x - nu_r) v[i - d_r] 1{x - nu_r in box} - a_r(x) v[i]).
-template <int R>
-__device__ __forceinline__ void accumulate(const Regs &g, const double *__restrict__ tab, const double *__restrict__ v,
-                                           int i, const int (&x)[NS], double vi, double &acc, double &dg) {
+template <int R, int L>  // reactions R, R + 1, .. that share leader L's net change
+__device__ __forceinline__ double gain_sum(const CufspBatchInst &in, const Tables &t, const int (&x)[NS]) {
     if constexpr (R < NR) {
-        double fa = g.coef[R], fb = g.coef[R];
-        bool ok = true;
-        src_factor<R, 0>(g, tab, x, fa, ok);
-        own_factor<R, 0>(g, tab, x, fb);
-        const double src = ok ? __ldg(v + i - g.delta[R]) : 0.0;
-        acc = fma(ok ? fa : 0.0, src, acc);
-        dg += fb;
-        accumulate<R + 1>(g, tab, v, i, x, vi, acc, dg);
+        if constexpr (leader(R) == L) {
+            const double f = first_used(R) < 0 ? in.coef[R] : gain_factor<R, 0>(in, t, x, 1.0);
+            if constexpr (R + 1 < NR) return f + gain_sum<R + 1, L>(in, t, x);
+            return f;
+        } else {
+            return gain_sum<R + 1, L>(in, t, x);
+        }
     }
+    return 0.0;
 }
 
-__device__ __forceinline__ void decode(const Regs &g, int i, int (&x)[NS]) {
-    unsigned rem = (unsigned)i;
-#pragma unroll
-    for (int sp = 0; sp < NS - 1; ++sp) {
-        const unsigned q = fdiv(rem, g.div[sp]);
-        x[sp] = (int)(rem - q * (unsigned)g.dims[sp]);
-        rem = q;
+template <int R, int SP>
+__device__ __forceinline__ double own_product(const CufspBatchInst &in, const double *__restrict__ tab, const int (&x)[NS],
+                                              double f) {
+    if constexpr (SP < NS) {
+        if constexpr (kind(R, SP) == 1) f *= (double)x[SP];
+        else if constexpr (kind(R, SP) == 2) f *= __ldg(tab + R * in.tab_stride + in.tab_off[SP] + x[SP]);
+        return own_product<R, SP + 1>(in, tab, x, f);
     }
-    x[NS - 1] = (int)rem;
+    return f;
+}
+
+template <int R>
+__device__ __forceinline__ void accumulate(const CufspBatchInst &in, const Tables &t, const double *__restrict__ tab,
+                                           const double *v, int i, const int (&x)[NS], double &acc, double &dg) {
+    if constexpr (R < NR) {
+        if constexpr (leader(R) == R)  // a source outside the box has gain 0; its index is kept in range
+            acc = fma(gain_sum<R, R>(in, t, x), v[min(max(i - in.delta[R], 0), in.n - 1)], acc);
+        if constexpr (own_species(R) == -1) dg += in.coef[R];
+        if constexpr (own_species(R) == -2) dg += own_product<R, 0>(in, tab, x, in.coef[R]);
+        accumulate<R + 1>(in, t, tab, v, i, x, acc, dg);
+    }
 }
 
 // rho * (A v)[i]
-__device__ __forceinline__ double apply_at(const Regs &g, const double *__restrict__ tab, const double *__restrict__ v,
-                                           int i, double rho) {
+__device__ __forceinline__ double apply_at(const CufspBatchInst &in, const Tables &t, const double *__restrict__ tab,
+                                           const double *v, int i, double rho) {
     int x[NS];
-    decode(g, i, x);
-    const double vi = __ldg(v + i);
+    unsigned rem = (unsigned)i;
+#pragma unroll
+    for (int sp = 0; sp < NS - 1; ++sp) {
+        const unsigned q = fdiv(rem, in.div[sp]);
+        x[sp] = (int)(rem - q * (unsigned)in.dims[sp]);
+        rem = q;
+    }
+    x[NS - 1] = (int)rem;
     double acc = 0.0, dg = 0.0;
-    accumulate<0>(g, tab, v, i, x, vi, acc, dg);
-    return rho * fma(-dg, vi, acc);
+#pragma unroll
+    for (int sp = 0; sp < NS; ++sp) dg += t.loss[in.tab_off[sp] + x[sp]];
+    accumulate<0>(in, t, tab, v, i, x, acc, dg);
+    return rho * fma(-dg, v[i], acc);
+}
+
+template <int R, int SP>
+__device__ __forceinline__ void fill_tables(const CufspBatchInst &in, const double *__restrict__ tab, double *gain,
+                                            double *loss) {
+    if constexpr (R < NR) {
+        if constexpr (SP < NS) {
+            const double *own = tab + R * in.tab_stride + in.tab_off[SP];
+            for (int x = threadIdx.x; x < in.dims[SP]; x += T) {
+                if constexpr (used(R, SP)) {
+                    const int y = x - nu(R, SP);
+                    double g = y < 0 || y >= in.dims[SP] ? 0.0 : kind(R, SP) == 0 ? 1.0 : __ldg(own + y);
+                    if (SP == first_used(R)) g *= in.coef[R];
+                    gain[R * in.tab_stride + in.tab_off[SP] + x] = g;
+                }
+                if constexpr (own_species(R) == SP) loss[in.tab_off[SP] + x] += in.coef[R] * __ldg(own + x);
+            }
+            fill_tables<R, SP + 1>(in, tab, gain, loss);
+        } else {
+            fill_tables<R + 1, 0>(in, tab, gain, loss);
+        }
+    }
+}
+
+// ---- a thread's states: pairs (i, i + 1), i even, 16 bytes a load -----------------------------------
+// Every basis vector starts on a 16-byte boundary (stride rounded up to even), so a pass over the chunk
+// keeps eight 16-byte loads per thread in flight: the passes over the basis are bound by how many bytes
+// are on their way from L2 and HBM.  With 8-byte loads (and four at a time in the update) 48 gene models
+// of 13K-113K states took @B0@ ms, so @B1@ ms.  The last state of an odd instance is a pair of one.
+__device__ __forceinline__ double2 ld2(const double *p, bool two) {
+    return two ? *reinterpret_cast<const double2 *>(p) : make_double2(*p, 0.0);
+}
+__device__ __forceinline__ void st2(double *p, double2 v, bool two) {
+    if (two) *reinterpret_cast<double2 *>(p) = v;
+    else *p = v.x;
+}
+template <class F>
+__device__ __forceinline__ void for_pairs(int i0, int i1, F &&f) {  // f(i, two)
+    int i = i0 + 2 * (int)threadIdx.x;
+#pragma unroll 1
+    for (; i + 1 < i1; i += 2 * T) f(i, true);
+    if (i < i1) f(i, false);
+}
+// the same from the end of the chunk
+template <class F>
+__device__ __forceinline__ void for_pairs_back(int i0, int i1, F &&f) {
+    const int pairs = (i1 - i0 + 1) >> 1, first = (int)threadIdx.x;
+    if (first >= pairs) return;
+    int i = i0 + 2 * (first + (pairs - 1 - first) / T * T);
+    if (i + 1 >= i1) {
+        f(i, false);
+        i -= 2 * T;
+    }
+#pragma unroll 1
+    for (; i >= i0; i -= 2 * T) f(i, true);
 }
 
 // Warp partial sums of up to 8 values into s.warp_part[warp][k0 + k].
@@ -248,30 +316,41 @@ __device__ void mm(const double *A, const double *B, double *C) {  // C = A B
     for (int e = threadIdx.x; e < MP2 * MP2; e += T) {
         const int i = e % MP2, j = e / MP2;
         double acc = 0.0;
+#pragma unroll 8
         for (int l = 0; l < MP2; ++l) acc = fma(A[i + l * MP2], B[l + j * MP2], acc);
         C[e] = acc;
     }
     __syncthreads();
 }
 
+__device__ __forceinline__ double nan_value() { return __longlong_as_double(0x7ff8000000000000ll); }
+
 // F = exp(A) by scaling and squaring Pade(13,13); false on NaN/Inf or a singular denominator.
 // Workspace: s.pade[0..7]; A is read from s.pade[7] and F is left in s.pade[0].
-__device__ bool expm_dev(Shared &s) {
+__device__ __noinline__ bool expm_dev(Shared &s) {
     double *A = s.pade[7];
     double *B = s.pade[0], *B2 = s.pade[1], *B4 = s.pade[2], *B6 = s.pade[3], *Tm = s.pade[4], *U = s.pade[5],
            *V = s.pade[6];
     __shared__ double norm1;
     __shared__ int sq;
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {  // 1-norm: a column per lane
         double nm = 0.0;
-        for (int j = 0; j < MP2; ++j) {
+        bool nan = false;
+        for (int j = threadIdx.x; j < MP2; j += 32) {
             double c = 0.0;
+#pragma unroll 4
             for (int i = 0; i < MP2; ++i) c += fabs(A[i + j * MP2]);
+            nan = nan || !isfinite(c);
             nm = fmax(nm, c);
         }
-        norm1 = nm;
-        const double theta13 = 5.371920351148152;
-        sq = (isfinite(nm) && nm > theta13) ? (int)ceil(log2(nm / theta13)) : 0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) nm = fmax(nm, __shfl_xor_sync(0xffffffffu, nm, o));
+        nan = __any_sync(0xffffffffu, nan);
+        if (threadIdx.x == 0) {
+            norm1 = nan ? nan_value() : nm;
+            const double theta13 = 5.371920351148152;
+            sq = (!nan && nm > theta13) ? (int)ceil(log2(nm / theta13)) : 0;
+        }
     }
     __syncthreads();
     if (!isfinite(norm1)) return false;
@@ -311,18 +390,29 @@ __device__ bool expm_dev(Shared &s) {
     if (threadIdx.x == 0) singular = 0;
     __syncthreads();
     for (int col = 0; col < MP2; ++col) {
-        if (threadIdx.x == 0) {
+        if (threadIdx.x < 32) {  // the first largest entry of the column on or below the diagonal
+            double best = -1.0;
             int p = col;
-            double best = fabs(P[col + col * MP2]);
-            for (int i = col + 1; i < MP2; ++i) {
+            for (int i = col + (int)threadIdx.x; i < MP2; i += 32) {
                 const double vv = fabs(P[i + col * MP2]);
                 if (vv > best) {
                     best = vv;
                     p = i;
                 }
             }
-            s.piv[col] = p;
-            if (best == 0.0) singular = 1;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+                const int op = __shfl_xor_sync(0xffffffffu, p, o);
+                if (ob > best || (ob == best && op < p)) {
+                    best = ob;
+                    p = op;
+                }
+            }
+            if (threadIdx.x == 0) {
+                s.piv[col] = p;
+                if (!(best > 0.0)) singular = 1;
+            }
         }
         __syncthreads();
         if (singular) return false;
@@ -353,15 +443,16 @@ __device__ bool expm_dev(Shared &s) {
         for (int i = col + 1 + threadIdx.x; i < MP2; i += T) P[i + col * MP2] *= inv;
         __syncthreads();
     }
-    // back substitution, one column of Q per thread group
-    for (int j = threadIdx.x; j < MP2; j += T) {
-        double *q = Q + j * MP2;
-        for (int c2 = MP2 - 1; c2 >= 0; --c2) {
-            q[c2] /= P[c2 + c2 * MP2];
-            for (int i = 0; i < c2; ++i) q[i] -= P[i + c2 * MP2] * q[c2];
+    // back substitution, a row of all columns at a time
+    for (int c2 = MP2 - 1; c2 >= 0; --c2) {
+        for (int j = threadIdx.x; j < MP2; j += T) Q[c2 + j * MP2] /= P[c2 + c2 * MP2];
+        __syncthreads();
+        for (int e = threadIdx.x; e < c2 * MP2; e += T) {
+            const int i = e % c2, j = e / c2;
+            Q[i + j * MP2] -= P[i + c2 * MP2] * Q[c2 + j * MP2];
         }
+        __syncthreads();
     }
-    __syncthreads();
     double *R = Q, *Tmp = B6;
     for (int k = 0; k < sq; ++k) {
         mm(R, R, Tmp);
@@ -369,16 +460,12 @@ __device__ bool expm_dev(Shared &s) {
         R = Tmp;
         Tmp = t0;
     }
-    for (int e = threadIdx.x; e < MP2 * MP2; e += T) s.pade[0][e] = R[e];
-    __syncthreads();
-    __shared__ int bad;
-    if (threadIdx.x == 0) {
-        bad = 0;
-        for (int e = 0; e < MP2 * MP2; ++e)
-            if (!isfinite(s.pade[0][e])) bad = 1;
+    bool bad = false;
+    for (int e = threadIdx.x; e < MP2 * MP2; e += T) {
+        s.pade[0][e] = R[e];
+        bad = bad || !isfinite(R[e]);
     }
-    __syncthreads();
-    return !bad;
+    return !__syncthreads_or(bad);
 }
 
 __device__ __forceinline__ double round2(double t) {
@@ -386,22 +473,126 @@ __device__ __forceinline__ double round2(double t) {
     return ceil(t / sc) * sc;
 }
 
+// ---- passes over the own chunk [i0, i1) of the states ---------------------------------------------
+// Called functions: each has the registers for its eight 16-byte loads, and what the solve keeps is
+// saved once per pass (inlined, 560 bytes a thread were spilled inside the loops of the 512-thread shape).
+// Basis vector k starts at v (k = 0) or W + (k - 1) ld.
+
+// w = rho A x, or (w null) the sum of squares of rho A x
+__device__ __noinline__ double pass_apply(const CufspBatchInst &in, const Tables &t, const double *tab, const double *x,
+                                          double *w, int i0, int i1, double rho) {
+    double acc = 0.0;
+    for_pairs(i0, i1, [&](int i, bool two) {
+        double2 r;
+        r.x = apply_at(in, t, tab, x, i, rho);
+        r.y = two ? apply_at(in, t, tab, x, i + 1, rho) : 0.0;
+        if (w) st2(w + i, r, two);
+        acc = fma(r.y, r.y, fma(r.x, r.x, acc));
+    });
+    return acc;
+}
+
+// Warp partial sums of W_k . w for the K vectors from k0 on
+__device__ __noinline__ void pass_dots(Shared &s, const double *v, const double *W, int ld, int k0, int K, const double *w,
+                                       int i0, int i1) {
+#pragma unroll 1
+    for (int g0 = 0; g0 < K; g0 += 8) {
+        double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        const int used = K - g0;
+        const double *const pn = W + (size_t)(k0 + g0) * ld, *const p0 = k0 + g0 == 0 ? v : pn - ld;
+        for_pairs(i0, i1, [&](int i, bool two) {
+            const double2 wi = ld2(w + i, two);
+            double2 x[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                x[k] = make_double2(0.0, 0.0);
+                if (k < used) x[k] = ld2((k ? pn + (k - 1) * ld : p0) + i, two);
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) acc[k] = fma(x[k].y, wi.y, fma(x[k].x, wi.x, acc[k]));
+        });
+        warp_partials8(s, acc, g0, K);
+    }
+}
+
+// w -= sum of c_k W_k over the K vectors from k0 on, returns the sum of squares of w.  Backwards: what
+// the dots have read last is still in L2 (15 bases of 14 MB do not fit it).
+__device__ __noinline__ double pass_update(const double *v, const double *W, int ld, int k0, int K, const double *c, double *w,
+                                           int i0, int i1) {
+    double acc = 0.0;
+    for_pairs_back(i0, i1, [&](int i, bool two) {
+        double2 r = ld2(w + i, two);
+#pragma unroll 1
+        for (int g0 = 0; g0 < K; g0 += 8) {
+            const double *const pn = W + (size_t)(k0 + g0) * ld + i, *const p0 = k0 + g0 == 0 ? v + i : pn - ld;
+            double2 x[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                x[k] = make_double2(0.0, 0.0);
+                if (g0 + k < K) x[k] = ld2(k ? pn + (k - 1) * ld : p0, two);
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const double ck = -c[g0 + k];  // past K: any finite number, times 0
+                r.x = fma(ck, x[k].x, r.x);
+                r.y = fma(ck, x[k].y, r.y);
+            }
+        }
+        st2(w + i, r, two);
+        acc = fma(r.y, r.y, fma(r.x, r.x, acc));
+    });
+    return acc;
+}
+
+// v = sum of c_k W_k over the first K vectors (W_0 = v: every pair is read before it is written)
+__device__ __noinline__ void pass_combine(double *v, const double *W, int ld, int K, const double *c, int i0, int i1) {
+    for_pairs(i0, i1, [&](int i, bool two) {
+        double2 r = make_double2(0.0, 0.0);
+#pragma unroll 1
+        for (int g0 = 0; g0 < K; g0 += 8) {
+            const double *const pn = W + (size_t)g0 * ld + i, *const p0 = g0 == 0 ? v + i : pn - ld;
+            double2 x[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                x[k] = make_double2(0.0, 0.0);
+                if (g0 + k < K) x[k] = ld2(k ? pn + (k - 1) * ld : p0, two);
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                r.x = fma(c[g0 + k], x[k].x, r.x);
+                r.y = fma(c[g0 + k], x[k].y, r.y);
+            }
+        }
+        st2(v + i, r, two);
+    });
+}
+
 // ---- one instance --------------------------------------------------------------------------
-__device__ void solve_instance(const CufspBatchArgs &a, cg::cluster_group &cl, Shared &s, double *__restrict__ W,
-                               int &buf) {
+__device__ void solve_instance(const CufspBatchArgs &a, cg::cluster_group &cl, Shared &s, double *W, double *tabs,
+                               int ld_max, int stride_max, int &buf) {
     const int n = s.in.n;
     const int nb = (int)cl.num_blocks(), rank = (int)cl.block_rank();
-    const int chunk = ((n + nb - 1) / nb + 31) & ~31;
+    const int chunk = ((n + nb - 1) / nb + 63) & ~63;
+    const int ld = (n + 1) & ~1;
     const int i0 = min(n, rank * chunk), i1 = min(n, i0 + chunk);
     double *v = a.p + s.in.off;
     const double *tab = a.tables + s.in.tab;
-    auto vec = [&](int k) -> double * { return k == 0 ? v : W + (size_t)(k - 1) * n; };
+    auto vec = [&](int k) -> double * { return k == 0 ? v : W + (size_t)(k - 1) * ld; };
     const double delta = 1.2, gamma = 0.9;
     double t_now = 0.0, t_new = 0.0, xm = 1.0 / M, err_loc = 0.0;
     const double btol = a.anorm * a.tol;
     int steps = 0, rejects = 0, matvecs = 0, status = 0;
-    Regs g;
-    load_regs(s.in, g);
+    Tables tb;
+    {  // each CTA its own tables: behind the solver's state in shared memory, or in the cluster's workspace
+        double *gain = CUFSP_BATCH_TABSMEM ? tabs : W + (size_t)(M + 1) * ld_max + (size_t)rank * (NR + 1) * stride_max;
+        double *loss = gain + NR * s.in.tab_stride;
+        for (int x = threadIdx.x; x < s.in.tab_stride; x += T) loss[x] = 0.0;
+        __syncthreads();
+        fill_tables<0, 0>(s.in, tab, gain, loss);
+        __syncthreads();
+        tb.gain = gain;
+        tb.loss = loss;
+    }
 
     while (t_now < a.t_final && status == 0) {
         if (steps >= a.max_steps) {
@@ -410,7 +601,10 @@ __device__ void solve_instance(const CufspBatchArgs &a, cg::cluster_group &cl, S
         }
         // beta = ||v||
         double acc1 = 0.0;
-        for (int i = i0 + (int)threadIdx.x; i < i1; i += T) acc1 = fma(v[i], v[i], acc1);
+        for_pairs(i0, i1, [&](int i, bool two) {
+            const double2 x = ld2(v + i, two);
+            acc1 = fma(x.y, x.y, fma(x.x, x.x, acc1));
+        });
         cluster_sum1(cl, s, acc1, buf);
         const double beta = sqrt(s.tot[0]);
         if (!isfinite(beta)) {
@@ -423,6 +617,7 @@ __device__ void solve_instance(const CufspBatchArgs &a, cg::cluster_group &cl, S
         }
         for (int e = threadIdx.x; e < MP2 * MP2; e += T) s.H[e] = 0.0;
         for (int e = threadIdx.x; e < MP2; e += T) s.rho[e] = 0.0;
+        for (int e = threadIdx.x; e < MP2 + 8; e += T) s.gam[e] = s.coefc[e] = 0.0;
         __syncthreads();
         if (threadIdx.x == 0) s.rho[0] = 1.0 / beta;
         __syncthreads();
@@ -439,30 +634,10 @@ __device__ void solve_instance(const CufspBatchArgs &a, cg::cluster_group &cl, S
             const double *vj = vec(j);
             double *w = vec(j + 1);
             const double rj = s.rho[j];
-            // generator action (own chunk; neighbours read anywhere in the instance)
-            for (int i = i0 + (int)threadIdx.x; i < i1; i += T) w[i] = apply_at(g, tab, vj, i, rj);
-            // Gram-Schmidt dots in groups of 8 (each thread re-reads only its own w entries)
-            for (int k0 = 0; k0 < K; k0 += 8) {
-                double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-                const double *vb[8];
-#pragma unroll
-                for (int k = 0; k < 8; ++k) vb[k] = vec(istart + min(k0 + k, K - 1));
-                if (K - k0 >= 8) {
-                    for (int i = i0 + (int)threadIdx.x; i < i1; i += T) {
-                        const double wi = w[i];
-#pragma unroll
-                        for (int k = 0; k < 8; ++k) acc[k] = fma(vb[k][i], wi, acc[k]);
-                    }
-                } else {
-                    for (int i = i0 + (int)threadIdx.x; i < i1; i += T) {
-                        const double wi = w[i];
-#pragma unroll
-                        for (int k = 0; k < 8; ++k)
-                            if (k0 + k < K) acc[k] = fma(vb[k][i], wi, acc[k]);
-                    }
-                }
-                warp_partials8(s, acc, k0, K);
-            }
+            // generator action (own chunk; neighbours read anywhere in the instance), Gram-Schmidt dots (each
+            // thread reads only its own w entries)
+            pass_apply(s.in, tb, tab, vj, w, i0, i1, rj);
+            pass_dots(s, v, W, ld, istart, K, w, i0, i1);
             cluster_finish(cl, s, K, buf);
             for (int k = threadIdx.x; k < K; k += T) {
                 const double h = s.rho[istart + k] * s.tot[k];
@@ -470,20 +645,7 @@ __device__ void solve_instance(const CufspBatchArgs &a, cg::cluster_group &cl, S
                 s.gam[istart + k] = h * s.rho[istart + k];
             }
             __syncthreads();
-            double acc2 = 0.0;
-            for (int i = i0 + (int)threadIdx.x; i < i1; i += T) {
-                double wi = w[i];
-                int k = 0;
-                for (; k + 4 <= K; k += 4) {
-                    wi = fma(-s.gam[istart + k], vec(istart + k)[i], wi);
-                    wi = fma(-s.gam[istart + k + 1], vec(istart + k + 1)[i], wi);
-                    wi = fma(-s.gam[istart + k + 2], vec(istart + k + 2)[i], wi);
-                    wi = fma(-s.gam[istart + k + 3], vec(istart + k + 3)[i], wi);
-                }
-                for (; k < K; ++k) wi = fma(-s.gam[istart + k], vec(istart + k)[i], wi);
-                w[i] = wi;
-                acc2 = fma(wi, wi, acc2);
-            }
+            const double acc2 = pass_update(v, W, ld, istart, K, s.gam + istart, w, i0, i1);
             cluster_sum1(cl, s, acc2, buf);
             const double sn = sqrt(s.tot[0]);
             ++matvecs;
@@ -511,11 +673,7 @@ __device__ void solve_instance(const CufspBatchArgs &a, cg::cluster_group &cl, S
         } else {  // avnorm = ||A v_m|| (src/KryExpvFSP.cu:114-120)
             const double *vm = vec(M);
             const double rm = s.rho[M];
-            double acc3 = 0.0;
-            for (int i = i0 + (int)threadIdx.x; i < i1; i += T) {
-                const double r = apply_at(g, tab, vm, i, rm);
-                acc3 = fma(r, r, acc3);
-            }
+            const double acc3 = pass_apply(s.in, tb, tab, vm, nullptr, i0, i1, rm);
             cluster_sum1(cl, s, acc3, buf);
             avnorm = sqrt(s.tot[0]);
             ++matvecs;
@@ -574,11 +732,7 @@ __device__ void solve_instance(const CufspBatchArgs &a, cg::cluster_group &cl, S
         mx = mb + max(0, k1 - 1);
         for (int k = threadIdx.x; k < mx; k += T) s.coefc[k] = beta * s.pade[0][k] * s.rho[k];
         __syncthreads();
-        for (int i = i0 + (int)threadIdx.x; i < i1; i += T) {
-            double r = 0.0;
-            for (int k = 0; k < mx; ++k) r = fma(s.coefc[k], vec(k)[i], r);
-            v[i] = r;
-        }
+        pass_combine(v, W, ld, mx, s.coefc, i0, i1);
         const bool last = tau >= a.t_final - t_now;
         t_now = last ? a.t_final : t_now + tau;
         if (err_loc > 0.0) t_new = round2(gamma * tau * pow(tau * a.tol / err_loc, xm));
@@ -624,7 +778,7 @@ extern "C" __global__ void __launch_bounds__(CUFSP_BATCH_THREADS, CUFSP_BATCH_MI
         for (int e = threadIdx.x; e < (int)(sizeof(CufspBatchInst) / sizeof(int)); e += T)
             reinterpret_cast<int *>(&s.in)[e] = reinterpret_cast<const int *>(a.inst + idx)[e];
         __syncthreads();
-        solve_instance(a, cl, s, W, buf);
+        solve_instance(a, cl, s, W, reinterpret_cast<double *>(dsm + sizeof(Shared)), a.ld_max, a.stride_max, buf);
         cl.sync();  // the cluster's workspace is free again
     }
 }
