@@ -103,6 +103,7 @@ struct Shared {
     double rho[MP2], gam[MP2 + 8];
     double pade[8][MP2 * MP2];  // exponential workspace
     double coefc[MP2 + 8];          // combination coefficients
+    double dpiv[MP2], dinv[MP2];  // pivots of the exponential's LU and their inverses
     int piv[MP2];
     CufspBatchInst in;          // current instance
     int inst_idx;
@@ -242,7 +243,7 @@ __device__ __forceinline__ void fill_tables(const CufspBatchInst &in, const doub
 // Every basis vector starts on a 16-byte boundary (stride rounded up to even), so a pass over the chunk
 // keeps eight 16-byte loads per thread in flight: the passes over the basis are bound by how many bytes
 // are on their way from L2 and HBM.  With 8-byte loads (and four at a time in the update) 48 gene models
-// of 13K-113K states took @B0@ ms, so @B1@ ms.  The last state of an odd instance is a pair of one.
+// of 13K-113K states took 104 ms, so (and with the tables below) 63 ms.  The last state of an odd instance is a pair of one.
 __device__ __forceinline__ double2 ld2(const double *p, bool two) {
     return two ? *reinterpret_cast<const double2 *>(p) : make_double2(*p, 0.0);
 }
@@ -250,10 +251,10 @@ __device__ __forceinline__ void st2(double *p, double2 v, bool two) {
     if (two) *reinterpret_cast<double2 *>(p) = v;
     else *p = v.x;
 }
-template <class F>
+template <int U, class F>  // U: pairs in flight per thread
 __device__ __forceinline__ void for_pairs(int i0, int i1, F &&f) {  // f(i, two)
     int i = i0 + 2 * (int)threadIdx.x;
-#pragma unroll 1
+#pragma unroll U
     for (; i + 1 < i1; i += 2 * T) f(i, true);
     if (i < i1) f(i, false);
 }
@@ -312,13 +313,18 @@ __device__ __forceinline__ void cluster_sum1(cg::cluster_group &cl, Shared &s, d
 }
 
 // ---- small dense kernels for the (m+2)^2 exponential (column-major, k = MP2) -------------------
-__device__ void mm(const double *A, const double *B, double *C) {  // C = A B
-    for (int e = threadIdx.x; e < MP2 * MP2; e += T) {
-        const int i = e % MP2, j = e / MP2;
-        double acc = 0.0;
+__device__ void mm(const double *A, const double *B, double *C) {  // C = A B, two columns per thread
+    for (int e = threadIdx.x; e < MP2 * ((MP2 + 1) / 2); e += T) {
+        const int i = e % MP2, j0 = e / MP2 * 2, j1 = min(j0 + 1, MP2 - 1);
+        double c0 = 0.0, c1 = 0.0;
 #pragma unroll 8
-        for (int l = 0; l < MP2; ++l) acc = fma(A[i + l * MP2], B[l + j * MP2], acc);
-        C[e] = acc;
+        for (int l = 0; l < MP2; ++l) {
+            const double al = A[i + l * MP2];
+            c0 = fma(al, B[l + j0 * MP2], c0);
+            c1 = fma(al, B[l + j1 * MP2], c1);
+        }
+        C[i + j0 * MP2] = c0;
+        C[i + j1 * MP2] = c1;
     }
     __syncthreads();
 }
@@ -384,8 +390,11 @@ __device__ __noinline__ bool expm_dev(Shared &s) {
         B4[e] = vv + u;  // Q = V + U (becomes the solution)
     }
     __syncthreads();
-    // LU with partial pivoting of P (B2), applied to Q (B4): one column per step.
+    // LU with partial pivoting of P (B2), applied to Q (B4): one column per step; a warp takes every WARPS-th
+    // column of [P Q], its lanes the rows (the other way round all lanes meet in one bank).
+    constexpr int RN = (MP2 + 31) / 32;  // rows per lane
     double *P = B2, *Q = B4;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     __shared__ int singular;
     if (threadIdx.x == 0) singular = 0;
     __syncthreads();
@@ -411,48 +420,62 @@ __device__ __noinline__ bool expm_dev(Shared &s) {
             }
             if (threadIdx.x == 0) {
                 s.piv[col] = p;
+                s.dpiv[col] = P[p + col * MP2];
+                s.dinv[col] = 1.0 / s.dpiv[col];
                 if (!(best > 0.0)) singular = 1;
             }
         }
         __syncthreads();
         if (singular) return false;
         const int p = s.piv[col];
-        if (p != col)
-            for (int j = threadIdx.x; j < MP2; j += T) {
-                double t0 = P[col + j * MP2];
-                P[col + j * MP2] = P[p + j * MP2];
-                P[p + j * MP2] = t0;
-                t0 = Q[col + j * MP2];
-                Q[col + j * MP2] = Q[p + j * MP2];
-                Q[p + j * MP2] = t0;
+        const double inv = s.dinv[col];
+        double l[RN];  // multipliers; rows p and col change places as the columns are read
+#pragma unroll
+        for (int q = 0; q < RN; ++q) {
+            const int i = lane + 32 * q;
+            l[q] = i > col && i < MP2 ? P[(i == p ? col : i) + col * MP2] * inv : 0.0;
+        }
+        for (int j = warp; j < 2 * MP2; j += WARPS) {
+            if (j <= col) continue;
+            double *c = j < MP2 ? P + j * MP2 : Q + (j - MP2) * MP2;
+            const double pivot = c[p], other = c[col];
+            double x[RN];
+#pragma unroll
+            for (int q = 0; q < RN; ++q) {
+                const int i = lane + 32 * q;
+                x[q] = i > col && i < MP2 ? fma(-l[q], pivot, i == p ? other : c[i]) : 0.0;
             }
-        __syncthreads();
-        const double inv = 1.0 / P[col + col * MP2];
-        // eliminate below the pivot in P (columns > col) and in every column of Q
-        for (int e = threadIdx.x; e < (MP2 - col - 1) * (2 * MP2); e += T) {
-            const int i = col + 1 + e % (MP2 - col - 1);
-            const int j = e / (MP2 - col - 1);
-            const double l = P[i + col * MP2] * inv;
-            if (j < MP2) {
-                if (j > col) P[i + j * MP2] -= l * P[col + j * MP2];
-            } else {
-                Q[i + (j - MP2) * MP2] -= l * Q[col + (j - MP2) * MP2];
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < RN; ++q) {
+                const int i = lane + 32 * q;
+                if (i > col && i < MP2) c[i] = x[q];
+                if (i == col) c[i] = pivot;
             }
         }
         __syncthreads();
-        for (int i = col + 1 + threadIdx.x; i < MP2; i += T) P[i + col * MP2] *= inv;
-        __syncthreads();
     }
-    // back substitution, a row of all columns at a time
-    for (int c2 = MP2 - 1; c2 >= 0; --c2) {
-        for (int j = threadIdx.x; j < MP2; j += T) Q[c2 + j * MP2] /= P[c2 + c2 * MP2];
-        __syncthreads();
-        for (int e = threadIdx.x; e < c2 * MP2; e += T) {
-            const int i = e % c2, j = e / c2;
-            Q[i + j * MP2] -= P[i + c2 * MP2] * Q[c2 + j * MP2];
-        }
-        __syncthreads();
+    // back substitution: a column of Q in the lanes of one warp
+    for (int j = warp; j < MP2; j += WARPS) {
+        double x[RN];
+#pragma unroll
+        for (int q = 0; q < RN; ++q) x[q] = lane + 32 * q < MP2 ? Q[lane + 32 * q + j * MP2] : 0.0;
+#pragma unroll
+        for (int q = RN - 1; q >= 0; --q)
+            for (int c2 = min(MP2, 32 * (q + 1)) - 1; c2 >= 32 * q; --c2) {
+                const double t = __shfl_sync(0xffffffffu, x[q], c2 & 31) / s.dpiv[c2];
+#pragma unroll
+                for (int r = 0; r <= q; ++r) {
+                    const int i = lane + 32 * r;
+                    if (i < c2) x[r] = fma(-P[i + c2 * MP2], t, x[r]);
+                    else if (i == c2) x[r] = t;
+                }
+            }
+#pragma unroll
+        for (int q = 0; q < RN; ++q)
+            if (lane + 32 * q < MP2) Q[lane + 32 * q + j * MP2] = x[q];
     }
+    __syncthreads();
     double *R = Q, *Tmp = B6;
     for (int k = 0; k < sq; ++k) {
         mm(R, R, Tmp);
@@ -480,9 +503,9 @@ __device__ __forceinline__ double round2(double t) {
 
 // w = rho A x, or (w null) the sum of squares of rho A x
 __device__ __noinline__ double pass_apply(const CufspBatchInst &in, const Tables &t, const double *tab, const double *x,
-                                          double *w, int i0, int i1, double rho) {
+                                          double *__restrict__ w, int i0, int i1, double rho) {
     double acc = 0.0;
-    for_pairs(i0, i1, [&](int i, bool two) {
+    for_pairs<1>(i0, i1, [&](int i, bool two) {
         double2 r;
         r.x = apply_at(in, t, tab, x, i, rho);
         r.y = two ? apply_at(in, t, tab, x, i + 1, rho) : 0.0;
@@ -500,7 +523,7 @@ __device__ __noinline__ void pass_dots(Shared &s, const double *v, const double 
         double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
         const int used = K - g0;
         const double *const pn = W + (size_t)(k0 + g0) * ld, *const p0 = k0 + g0 == 0 ? v : pn - ld;
-        for_pairs(i0, i1, [&](int i, bool two) {
+        for_pairs<1>(i0, i1, [&](int i, bool two) {
             const double2 wi = ld2(w + i, two);
             double2 x[8];
 #pragma unroll
@@ -546,7 +569,7 @@ __device__ __noinline__ double pass_update(const double *v, const double *W, int
 
 // v = sum of c_k W_k over the first K vectors (W_0 = v: every pair is read before it is written)
 __device__ __noinline__ void pass_combine(double *v, const double *W, int ld, int K, const double *c, int i0, int i1) {
-    for_pairs(i0, i1, [&](int i, bool two) {
+    for_pairs<1>(i0, i1, [&](int i, bool two) {
         double2 r = make_double2(0.0, 0.0);
 #pragma unroll 1
         for (int g0 = 0; g0 < K; g0 += 8) {
@@ -601,7 +624,7 @@ __device__ void solve_instance(const CufspBatchArgs &a, cg::cluster_group &cl, S
         }
         // beta = ||v||
         double acc1 = 0.0;
-        for_pairs(i0, i1, [&](int i, bool two) {
+        for_pairs<1>(i0, i1, [&](int i, bool two) {
             const double2 x = ld2(v + i, two);
             acc1 = fma(x.y, x.y, fma(x.x, x.x, acc1));
         });
