@@ -187,6 +187,18 @@ void launch_mdot_grouped(const MVecArgs &a, int mode, int sm_count, cudaStream_t
     else k_mdot_grouped<KG, G, false><<<4 * sm_count, kRedThreads, 0, st>>>(a);
 }
 
+// What follows from s = ||W_{j+1}||.
+__device__ __forceinline__ void finish_norm(const MVecArgs &a, double sn) {
+    if (!isfinite(sn)) {
+        *a.s.flag = -1;
+    } else if (sn < *a.s.btol) {
+        *a.s.flag = a.j + 1;
+    } else {
+        a.s.H[(a.j + 1) + a.j * a.s.mp2] = sn;
+        a.s.rho[a.j + 1] = 1.0 / sn;
+    }
+}
+
 // W_{j+1} -= sum_k gam_k W_k;  s = rho_j-scaled norm;  H(j+1, j) = s;  rho_{j+1} = 1/s;
 // happy breakdown when s < btol (src/KryExpvFSP.cu:76-105).
 template <int KP>
@@ -207,17 +219,129 @@ __global__ void __launch_bounds__(kRedThreads) k_mupd(const MVecArgs a) {
         acc[0] = fma(wi, wi, acc[0]);
     }
     if (!grid_reduce<1>(acc, 1, a.partials, a.counter, sm)) return;
-    if (threadIdx.x == 0) {
-        const double sn = sqrt(sm.final_[0]);
-        if (!isfinite(sn)) {
-            *a.s.flag = -1;
-        } else if (sn < *a.s.btol) {
-            *a.s.flag = a.j + 1;
-        } else {
-            a.s.H[(a.j + 1) + a.j * a.s.mp2] = sn;
-            a.s.rho[a.j + 1] = 1.0 / sn;
+    if (threadIdx.x == 0) finish_norm(a, sqrt(sm.final_[0]));
+}
+
+// ---- the same two passes on pairs of states, 16 bytes a load ---------------------------------------
+// For vectors of an even number of states on 16-byte boundaries (pairs_ok).  Both passes are bound by
+// HBM; what they need is bytes on their way.  A thread keeps eight 16-byte loads in flight: KG (KB) basis
+// vectors of U pairs, U = 2 where the window has at most four vectors (incomplete orthogonalisation),
+// whose three or four 8-byte loads of one state left the memory idle.  The update walks the vectors
+// backwards: the ends, which the dots have read last, are still in L2 (126 MB).
+// Measured, 5.5M states, window of 3 (IOP): dots 36 -> 33.6 us, update 49 -> 38.7 us (cold L2); 16.8M states, K = 30:
+// dots 613 us and update 621 us, 6.8 and 6.9 TB/s; a step of m = 30 there 24.38 -> 24.04 ms.
+template <int KG, int G, int U>
+__global__ void __launch_bounds__(kRedThreads, 3) k_mdot_pairs(const MVecArgs a) {
+    constexpr int KP = KG * G;
+    constexpr int S = kRedWarps / G;  // slices of 32 pairs in a CTA tile
+    static_assert(S * G == kRedWarps, "G must divide the warps of a CTA");
+    __shared__ RedSmem<KP> sm;
+    if (*a.s.flag) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g = warp % G, slice = warp / G;
+    const int Kb = (a.K + G - 1) / G, k0 = g * Kb;
+    const int Kg = max(0, min(Kb, a.K - k0));
+    const int ka = a.kbase + k0;
+    const int64_t np = a.n >> 1;
+    const double2 *const p_next = reinterpret_cast<const double2 *>(a.W) + (int64_t)ka * np;  // vector ka + 1
+    const double2 *const p_first = ka == 0 ? reinterpret_cast<const double2 *>(a.v0) : p_next - np;
+    const double2 *const pw = reinterpret_cast<const double2 *>(a.w);
+    double acc[KG];
+#pragma unroll
+    for (int k = 0; k < KG; ++k) acc[k] = 0.0;
+    const int64_t stride = (int64_t)gridDim.x * S * 32;
+    for (int64_t i0 = ((int64_t)blockIdx.x * S + slice) * 32 + lane; i0 < np; i0 += U * stride) {
+        double2 w[U], x[U][KG];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int64_t i = i0 + u * stride;
+            const bool in = i < np;
+            w[u] = in ? __ldg(pw + i) : make_double2(0.0, 0.0);
+#pragma unroll
+            for (int k = 0; k < KG; ++k) {
+                x[u][k] = make_double2(0.0, 0.0);
+                if (in && k < Kg) x[u][k] = __ldg((k ? p_next + (k - 1) * np : p_first) + i);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int k = 0; k < KG; ++k) acc[k] = fma(x[u][k].y, w[u].y, fma(x[u][k].x, w[u].x, acc[k]));
+    }
+#pragma unroll
+    for (int k = 0; k < KG; ++k) {
+        if (k < Kg) {
+            double v = acc[k];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0) sm.warp_part[warp][k] = v;
         }
     }
+    __syncthreads();
+    for (int k = threadIdx.x; k < a.K; k += blockDim.x) {
+        const int gg = k / Kb, kk = k - gg * Kb;
+        double v = 0.0;
+        for (int s = 0; s < S; ++s) v += sm.warp_part[s * G + gg][kk];
+        a.partials[(size_t)blockIdx.x * KP + k] = v;
+    }
+    if (!grid_finish<KP>(a.K, a.partials, a.counter, sm)) return;
+    for (int k = threadIdx.x; k < a.K; k += blockDim.x) {
+        const int kk = a.kbase + k;
+        const double r = a.s.rho[kk];
+        const double h = r * sm.final_[k];
+        a.s.H[kk + a.j * a.s.mp2] = h;
+        a.s.gam[kk] = h * r;
+    }
+}
+
+template <int KB, int U>
+__global__ void __launch_bounds__(kRedThreads, 3) k_mupd_pairs(const MVecArgs a) {
+    __shared__ RedSmem<1> sm;
+    __shared__ double g[kMaxVec + 8];
+    if (*a.s.flag) return;
+    for (int k = threadIdx.x; k < kMaxVec + 8; k += blockDim.x) g[k] = k < a.K ? a.s.gam[a.kbase + k] : 0.0;
+    __syncthreads();
+    const int64_t np = a.n >> 1;
+    const double2 *const Wb = reinterpret_cast<const double2 *>(a.W) + (int64_t)a.kbase * np;  // vector kbase + 1
+    const double2 *const p_first = a.kbase == 0 ? reinterpret_cast<const double2 *>(a.v0) : Wb - np;
+    double2 *const pw = reinterpret_cast<double2 *>(a.w);
+    double acc[1] = {0.0};
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < np; i0 += U * stride) {
+        double2 w[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) w[u] = i0 + u * stride < np ? pw[np - 1 - i0 - u * stride] : make_double2(0.0, 0.0);
+#pragma unroll 1
+        for (int k0 = 0; k0 < a.K; k0 += KB) {
+            double2 x[U][KB];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int64_t i = np - 1 - i0 - u * stride;
+#pragma unroll
+                for (int k = 0; k < KB; ++k) {
+                    x[u][k] = make_double2(0.0, 0.0);
+                    if (i >= 0 && k0 + k < a.K) x[u][k] = __ldg((k0 + k ? Wb + (int64_t)(k0 + k - 1) * np : p_first) + i);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int k = 0; k < KB; ++k) {
+                    w[u].x = fma(-g[k0 + k], x[u][k].x, w[u].x);
+                    w[u].y = fma(-g[k0 + k], x[u][k].y, w[u].y);
+                }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int64_t i = np - 1 - i0 - u * stride;
+            if (i >= 0) {
+                pw[i] = w[u];
+                acc[0] = fma(w[u].y, w[u].y, fma(w[u].x, w[u].x, acc[0]));
+            }
+        }
+    }
+    if (!grid_reduce<1>(acc, 1, a.partials, a.counter, sm)) return;
+    if (threadIdx.x == 0) finish_norm(a, sqrt(sm.final_[0]));
 }
 
 // avnorm = ||A v_m|| (src/KryExpvFSP.cu:114-120); skipped after a breakdown.
@@ -328,6 +452,11 @@ int mdot_mode() {
     return mode;
 }
 
+// Every vector starts on a 16-byte boundary and has no odd state left over.
+bool pairs_ok(const cufsp_expv *E, const double *v) {
+    return E->n % 2 == 0 && ((reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(E->W)) & 15) == 0;
+}
+
 template <int KP>
 void launch_mdot(const MVecArgs &a, int grid, cudaStream_t st) { k_mdot<KP><<<grid, kRedThreads, 0, st>>>(a); }
 template <int KP>
@@ -351,6 +480,19 @@ cufsp_status arnoldi_dot_update(cufsp_expv *E, double *v, int j, int istart, cud
     const int K = a.K;
     const int mode = mdot_mode();
     const int sms = device_info().sm_count;
+    if (mode == 2 && E->grid >= 4 * sms && pairs_ok(E, v)) {
+        const int g = 3 * sms;
+        if (K <= 4) k_mdot_pairs<4, 1, 2><<<g, kRedThreads, 0, st>>>(a);
+        else if (K <= 8) k_mdot_pairs<8, 1, 1><<<g, kRedThreads, 0, st>>>(a);
+        else if (K <= 16) k_mdot_pairs<8, 2, 1><<<g, kRedThreads, 0, st>>>(a);
+        else if (K <= 32) k_mdot_pairs<8, 4, 1><<<g, kRedThreads, 0, st>>>(a);
+        else k_mdot_pairs<8, 8, 1><<<g, kRedThreads, 0, st>>>(a);
+        CUFSP_CUDA_TRY(cudaGetLastError());
+        if (K <= 4) k_mupd_pairs<4, 2><<<g, kRedThreads, 0, st>>>(a);
+        else k_mupd_pairs<8, 1><<<g, kRedThreads, 0, st>>>(a);
+        CUFSP_CUDA_TRY(cudaGetLastError());
+        return CUFSP_SUCCESS;
+    }
     if (mode == 0 || E->grid < 4 * sms) {  // small vectors: the grid of the other pass kernels
         if (K <= 8) launch_mdot<8>(a, E->grid, st);
         else if (K <= 16) launch_mdot<16>(a, E->grid, st);
