@@ -197,15 +197,15 @@ void launch_adj_bilinear(const BilinArgs &ba, int grid, cudaStream_t st) {
     else k_adj_bilinear<32><<<grid, kRedThreads, 0, st>>>(ba);
 }
 
-// beta * exp(s H) e1 for an mb x mb column-major H (host).
+// beta * exp(s H) e1 for an mb x mb column-major upper Hessenberg H (host).
 cufsp_status dense_output(int mb, const std::vector<double> &H, double s, double beta, std::vector<double> &y) {
     y.assign(mb, 0.0);
     if (mb == 0) return CUFSP_SUCCESS;
-    std::vector<double> X((size_t)mb * mb), F((size_t)mb * mb);
+    std::vector<double> X((size_t)mb * mb);
     for (size_t i = 0; i < X.size(); ++i) X[i] = s * H[i];
-    cufsp_status st = expm_pade13(mb, X.data(), F.data());
+    cufsp_status st = expm_hessenberg_col(mb, X.data(), y.data());
     if (st != CUFSP_SUCCESS) return st;
-    for (int i = 0; i < mb; ++i) y[i] = beta * F[i];
+    for (int i = 0; i < mb; ++i) y[i] *= beta;
     return CUFSP_SUCCESS;
 }
 

@@ -766,7 +766,7 @@ cufsp_status expv_step(cufsp_expv *E, double *v, cudaStream_t st) {
     while (ireject < E->max_reject) {  // rejection loop, :122-158
         const int mx = mb + k1;
         for (int i = 0; i < mp2 * mp2; ++i) E->tH[i] = tau * E->Hh[i];
-        s = expm_pade13(mp2, E->tH.data(), E->F.data());
+        s = expm_hessenberg_col(mp2, E->tH.data(), E->F.data());
         if (s != CUFSP_SUCCESS) return s;
         if (k1 == 0) {
             err_loc = E->btol;
