@@ -65,6 +65,9 @@ struct PArgs {
     double *ex_next;            // that of the next launch, set back to unset here
     int ex_rows;                // rows of an area
     int *err;                   // set when a wait expired
+    double *h_state;            // pinned host copy of the state block (nullable), its length and sequence word
+    int words;
+    unsigned *h_seq, seq;
 };
 
 struct PSmem {
@@ -251,6 +254,13 @@ __global__ void __launch_bounds__(NT, 1) k_arnoldi_persistent(const __grid_const
                         if (!isfinite(av)) *a.flag = -1;
                     }
                 }
+            }
+            if (blockIdx.x == 0 && a.h_state) {  // to the host: all of it was written by this CTA
+                __syncthreads();
+                for (int i = tid; i < a.words; i += NT) a.h_state[i] = a.H[i];
+                __threadfence_system();
+                __syncthreads();
+                if (tid == 0) *(volatile unsigned *)a.h_seq = a.seq;
             }
             return;
         }
@@ -598,7 +608,7 @@ cudaError_t persistent_smem_attribute() {
 cufsp_status parnoldi_run(PArnoldi **ppa, cufsp_mat *A, const std::vector<double> &coefs, bool transpose,
                           int64_t n, const double *v, double *W, double *H, double *rho, double *gam, double *beta,
                           double *avnorm, int *flag, int *err, int m, int iop, int q, double btol, bool with_avnorm,
-                          cudaStream_t st) {
+                          double *h_state, int words, unsigned *h_seq, unsigned seq, cudaStream_t st) {
     if (!*ppa) *ppa = new PArnoldi();
     PArnoldi *pa = *ppa;
     PArnoldi::Terms *tm = nullptr;
@@ -674,6 +684,10 @@ cufsp_status parnoldi_run(PArnoldi **ppa, cufsp_mat *A, const std::vector<double
     a.ex_next = pa->d_ex + (size_t)(1 - pa->turn) * area;
     a.ex_rows = pa->ex_rows;
     a.err = err;
+    a.h_state = h_state;
+    a.words = words;
+    a.h_seq = h_seq;
+    a.seq = seq;
     pa->turn = 1 - pa->turn;
     a.terms.n = (int)n;
     split_terms(a.T, a.shift, a.terms);

@@ -576,7 +576,8 @@ bool spin_state() {
     return on;
 }
 
-cufsp_status fetch_state(cufsp_expv *E, cudaStream_t st) {
+// Makes this thread's pinned block hold E's state; false when it cannot (or CUFSP_KRYLOV_SPIN=0).
+bool pin_ready(cufsp_expv *E) {
     bool spin = spin_state();
     if (spin && tl_pin.bytes < E->state_bytes) {
         if (tl_pin.p) cudaFreeHost(tl_pin.p);
@@ -594,15 +595,23 @@ cufsp_status fetch_state(cufsp_expv *E, cudaStream_t st) {
             spin = false;
         }
     }
-    if (!spin) {
+    return spin;
+}
+
+// published: a kernel on st already copies the block and raises the word to tl_pin.n.
+cufsp_status fetch_state(cufsp_expv *E, cudaStream_t st, bool published) {
+    if (!published && !pin_ready(E)) {
         CUFSP_CUDA_TRY(cudaMemcpyAsync(E->hstate.data(), E->d_state, E->state_bytes, cudaMemcpyDeviceToHost, st));
         CUFSP_CUDA_TRY(cudaStreamSynchronize(st));
         return CUFSP_SUCCESS;
     }
-    const unsigned seq = ++tl_pin.n;
-    const int words = (int)(E->state_bytes / sizeof(double));
-    k_publish_state<<<1, 256, 0, st>>>(E->d_state, tl_pin.p, words, tl_pin.seq, seq);
-    CUFSP_CUDA_TRY(cudaGetLastError());
+    if (!published) {
+        ++tl_pin.n;
+        const int words = (int)(E->state_bytes / sizeof(double));
+        k_publish_state<<<1, 256, 0, st>>>(E->d_state, tl_pin.p, words, tl_pin.seq, tl_pin.n);
+        CUFSP_CUDA_TRY(cudaGetLastError());
+    }
+    const unsigned seq = tl_pin.n;
     const auto t0 = std::chrono::steady_clock::now();
     for (unsigned it = 1; *(volatile unsigned *)tl_pin.seq != seq; ++it) {
         if ((it & 1023) == 0) {
@@ -610,7 +619,13 @@ cufsp_status fetch_state(cufsp_expv *E, cudaStream_t st) {
             if (std::chrono::steady_clock::now() - t0 > std::chrono::seconds(10)) break;
         }
     }
-    if (*(volatile unsigned *)tl_pin.seq != seq) CUFSP_CUDA_TRY(cudaStreamSynchronize(st));
+    if (*(volatile unsigned *)tl_pin.seq != seq) {
+        CUFSP_CUDA_TRY(cudaStreamSynchronize(st));
+        if (*(volatile unsigned *)tl_pin.seq != seq) {  // a persistent pass that broke off: the block as it stands
+            CUFSP_CUDA_TRY(cudaMemcpy(E->hstate.data(), E->d_state, E->state_bytes, cudaMemcpyDeviceToHost));
+            return CUFSP_SUCCESS;
+        }
+    }
     std::memcpy(E->hstate.data(), tl_pin.p, E->state_bytes);
     return CUFSP_SUCCESS;
 }
@@ -635,10 +650,12 @@ cufsp_status arnoldi_pass(cufsp_expv *E, double *v, cudaStream_t st, bool with_a
     E->used = true;
     E->last_stream = st;
     const bool persistent = E->A && parnoldi_wanted(E->A, E->n, E->m);
+    const bool published = persistent && pin_ready(E);  // the pass copies the state block itself
     if (persistent) {
         s = parnoldi_run(&E->pa, E->A, E->coefs, E->transpose, E->n, v, E->W, E->ks.H, E->ks.rho, E->ks.gam,
                          E->ks.beta, E->ks.avnorm, E->ks.flag, E->ks.flag + 1, E->m, E->iop, E->q_iop, btol_eff,
-                         with_avnorm, st);
+                         with_avnorm, published ? tl_pin.p : nullptr, (int)(E->state_bytes / sizeof(double)), tl_pin.seq,
+                         published ? ++tl_pin.n : 0, st);
         if (s != CUFSP_SUCCESS) return s;
     } else if (E->A && graphs_enabled()) {
         *E->h_btol = btol_eff;  // the previous pass's copy has completed: the stream was synchronised after it
@@ -676,7 +693,7 @@ cufsp_status arnoldi_pass(cufsp_expv *E, double *v, cudaStream_t st, bool with_a
         if (s != CUFSP_SUCCESS) return s;
     }
     const int m = E->m;
-    s = fetch_state(E, st);
+    s = fetch_state(E, st, published);
     if (s != CUFSP_SUCCESS) return s;
     // basis data for the adjoint (leading mb x mb block of H, rho, beta)
     const int mp2 = m + 2;
@@ -806,7 +823,8 @@ cufsp_status expv_step(cufsp_expv *E, double *v, cudaStream_t st) {
         c.vec[k] = wvec(E, v, k);
         c.c[k] = beta * E->F[k] * hrho[k];
     }
-    const int g = stream_grid(E->n, 4, device_info().sm_count * 8);
+    // (one state per thread while the GPU is not full: at 32,768 states four left it to 32 CTAs)
+    const int g = stream_grid(E->n, 1, device_info().sm_count * 8);
     if (mx <= 8) launch_comb<8>(c, g, st);
     else if (mx <= 16) launch_comb<16>(c, g, st);
     else if (mx <= 32) launch_comb<32>(c, g, st);

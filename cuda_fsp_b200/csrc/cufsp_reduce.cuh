@@ -46,6 +46,7 @@ __device__ __forceinline__ bool grid_finish(int K, double *__restrict__ partials
         double v = 0.0;
         if (k < K) {
             const volatile double *vp = partials;
+#pragma unroll 8
             for (int c = g; c < (int)gridDim.x; c += G) v += vp[(size_t)c * KP + k];
         }
         grp[g * KP + k] = v;
