@@ -17,12 +17,12 @@
 //  * the generator is applied from a per-state term table built once per coefficient vector:
 //      (A x)[i] = sum_t coef[t][i] x[i - shift_t]   (last term: shift 0, the diagonal),
 //    coefficient 0 wherever the source state leaves the box (its index is clamped to [0, n)).  A CTA
-//    owns a contiguous slice of the states; up to 2 states per thread and 12 terms the coefficients stay
-//    in registers for the whole launch, and sources inside the slice come from shared memory.
+//    owns a contiguous slice of the states; up to 4 states per thread, 10 near and 8 far terms the coefficients
+//    stay in registers for the whole launch, and sources inside the slice come from shared memory.
 //  * the CTA's slices of as many basis vectors as fit live in shared memory (all 30 of them up to 148 x
 //    ~890 = 131K states); the dots and the update read them there and the rest from L2.
 // Measured, a Krylov step of m = 30 (pass, host step control and combination): 32,768 states 0.35 ms with
-// two barriers per iteration, 0.20 ms so; 134,088 states 0.50 and 0.28 ms.
+// two barriers per iteration, 0.19 ms so; 134,088 states 0.50 and 0.26 ms.
 // Waits are bounded; on expiry the kernel sets an error word, every CTA leaves, and the host reports
 // CUFSP_ERR_CUDA.  The launch is cooperative, so all CTAs are co-resident.
 #include <algorithm>
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(NT, 1) k_arnoldi_persistent(const __grid_const
         if (!last || a.with_avnorm) {
             if constexpr (REG) {
                 double v[NS][TF];
-                bad = !gather_begin<NT, NS, TF>(a.terms, x, lo, len, j > 0, xs, v, a.err);
+                bad = !gather_begin<NT, NS, TF, false>(a.terms, x, lo, len, j > 0, xs, v, a.err);
                 __syncthreads();
                 if (!gather_end<NT, NS, TN, TF>(a.terms, x, lo, len, j > 0, xs, cn, cfar, v, w, a.err)) bad = true;
 #pragma unroll

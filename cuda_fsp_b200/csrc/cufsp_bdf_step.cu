@@ -1,5 +1,5 @@
 // cufsp_bdf_step.cu -- one step attempt of the BDF integrator (cufsp_bdf.cu) as ONE persistent launch,
-// for generators whose slices fit the CTAs' registers and shared memory (up to 148 x 1024 states).
+// for generators whose slices fit the CTAs' registers and shared memory (up to 148 x 1056 = 156,288 states).
 //
 // The launch sequence spends a step on some 60 launches and 8 waits of the host for scalars: 344 us a step
 // on the 131,072-state gene model (5.4 GMRES iterations), nearly all of it launch and round-trip latency.
@@ -20,7 +20,7 @@
 // published vectors in L2).  An extra warp collects totals and runs the Givens rotations beside the
 // update.  What bounds it is the chain of exchanges, two and one gather per iteration (cufsp_grid.cuh).
 // Measured on the 131,072-state gene model to t = 6 (315 steps): 0.34 ms a step with the launch
-// sequence, 0.090 ms so.
+// sequence, 0.088 ms so.
 // The coefficients c_r(t_new): tables of unit propensities, gain and outflow, are built once per
 // generator, a table of the terms' coefficients from them for the reactions with constant rates; the
 // launch adds the reactions whose rates have changed.  Waits are bounded; on expiry the error word is set and every CTA leaves.
@@ -211,8 +211,7 @@ __global__ void __launch_bounds__(kThreads + 32, 1) k_bdf_step(const __grid_cons
         acc = 0.0;
         {
             double v[NS][TF];
-            if (work) bad = !gather_begin<NT, NS, TF>(a.terms, x, lo, len, true, xs, v, a.err);
-            __syncthreads();
+            if (work) bad = !gather_begin<NT, NS, TF, true>(a.terms, x, lo, len, true, xs, v, a.err);
             if (work && !gather_end<NT, NS, TN, TF>(a.terms, x, lo, len, true, xs, cn, cf, v, q, a.err)) bad = true;
         }
         if (J < 0) {
