@@ -228,7 +228,11 @@ __global__ void __launch_bounds__(kRedThreads) k_mupd(const MVecArgs a) {
 // vectors of U pairs, U = 2 where the window has at most four vectors (incomplete orthogonalisation),
 // whose three or four 8-byte loads of one state left the memory idle.  The update walks the vectors
 // backwards: the ends, which the dots have read last, are still in L2 (126 MB).
-// Measured, 5.5M states, window of 3 (IOP): dots 36 -> 33.6 us, update 49 -> 38.7 us (cold L2); 16.8M states, K = 30:
+// With at most four vectors the update reads the oldest with the evict-first hint: it leaves the window, and
+// the L2 lines it gives up keep what the generator and the next dots read (one iteration, window of 3: 5.5M
+// states 110.7 -> 107.7 us, 2.6M states 55.8 -> 53.2 us, 16.8M states 340 -> 333 us).  The dots backwards and
+// the update forwards would take 113 us at 5.5M states, stores of the generator without their hint 109.0 us.
+// Measured, 5.5M states, window of 3 (IOP): dots 36 -> 33.6 us, update 49 -> 38.7 us (cold L2, without the hint); 16.8M states, K = 30:
 // dots 613 us and update 621 us, 6.8 and 6.9 TB/s; a step of m = 30 there 24.38 -> 24.04 ms.
 template <int KG, int G, int U>
 __global__ void __launch_bounds__(kRedThreads, 3) k_mdot_pairs(const MVecArgs a) {
@@ -320,7 +324,8 @@ __global__ void __launch_bounds__(kRedThreads, 3) k_mupd_pairs(const MVecArgs a)
 #pragma unroll
                 for (int k = 0; k < KB; ++k) {
                     x[u][k] = make_double2(0.0, 0.0);
-                    if (i >= 0 && k0 + k < a.K) x[u][k] = __ldg((k0 + k ? Wb + (int64_t)(k0 + k - 1) * np : p_first) + i);
+                    if (i >= 0 && k0 + k < a.K)
+                        x[u][k] = U == 2 && k == 0 ? __ldcs(p_first + i) : __ldg((k0 + k ? Wb + (int64_t)(k0 + k - 1) * np : p_first) + i);
                 }
             }
 #pragma unroll
