@@ -507,17 +507,23 @@ extern "C" cufsp_status cufsp_likelihood_grad_batched(const cufsp_model_desc *de
         return set_error(CUFSP_ERR_INVALID_ARG, "cufsp_likelihood_grad_batched: bad argument");
     const int nr = desc->n_reactions;
     workers = std::max(1, std::min(std::min(workers, n_sets), 32));
-    // Generators small enough for the persistent Arnoldi pass: every worker's passes take an equal
-    // share of the SMs (CUFSP_GRAD_SM_SHARE=0: each pass takes all SMs and the passes of the workers
-    // take turns), so that the workers' solves run side by side; larger generators run `workers`
-    // concurrent launch sequences.
+    // Generators small enough for the persistent Arnoldi pass: up to kShareStates states per SM every
+    // worker's passes take an equal share of the SMs, so that the workers' solves run side by side; above,
+    // a share's slices of the basis would no longer fit its shared memory, and each pass takes all SMs, the
+    // passes of two workers in turn (one's host work beside the other's pass).  Gradients/s of 16 sets, 4 workers
+    // asked for, shares and turns: 64,800 states 5.97 and 5.11, 93,312 states (630 per SM) 4.36 and 4.21,
+    // 131,072 states (886 per SM) 2.55 and 3.11.
+    // CUFSP_GRAD_SM_SHARE=0 or 1: always turns, always shares.  Larger generators run `workers` concurrent
+    // launch sequences.
+    constexpr int64_t kShareStates = 700;
     int64_t n_states = 1;
     for (int s = 0; s < desc->n_species; ++s) n_states *= (int64_t)desc->fsp_bounds[s] + 1;
     const bool persistent = parnoldi_size_ok(n_states);
+    const int sms = device_info().sm_count;
     const char *share_env = getenv("CUFSP_GRAD_SM_SHARE");
-    const bool share = !share_env || atoi(share_env) != 0;
+    const bool share = share_env ? atoi(share_env) != 0 : n_states <= kShareStates * sms;
     int cta_cap = 0;
-    if (persistent && share) cta_cap = std::max(1, device_info().sm_count / workers);
+    if (persistent && share) cta_cap = std::max(1, sms / workers);
     else if (persistent) workers = std::min(workers, 2);
     int dev = 0;
     CUFSP_CUDA_TRY(cudaGetDevice(&dev));
