@@ -20,7 +20,8 @@
 // Registers limit an SM to 16 warps, whose loads of one chunk of reactions do not cover the DRAM latency:
 // a CTA therefore first asks L2 for all rows of its tile, one bulk prefetch per row by one thread each
 // (row r where it is first touched: at the source when the source lies ahead).  9 reactions: 160 x 151 x
-// 132 states 61.7 -> 59.7 us, 256^3 275 -> 271 us; 12 reactions, 0.9M states 25.9 -> 24.9 us.  Asking for
+// 132 states 61.7 -> 59.7 us (63.2 -> 63.0 us after another generator), 256^3 275 -> 271 us; 12 reactions,
+// 0.9M states 25.9 -> 24.9 us.  Asking for
 // the tile after that, or the next two, costs more than it hides (61.0, 63.6 us; 312, 333 us): the rows
 // that are read again at their sources leave L2 sooner.
 #ifndef CUFSP_SPARSE_RTC_CUH
