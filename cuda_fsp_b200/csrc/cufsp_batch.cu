@@ -222,7 +222,7 @@ struct cufsp_batch_s {
     unsigned *d_counter = nullptr;
     double *d_work = nullptr;
     size_t work_doubles = 0;
-    double *d_scratch = nullptr;           // autotuner trial vectors
+    double *d_scratch = nullptr;           // autotuner trial vectors, aligned copy of the caller's vectors
     // chosen launch shape
     int cluster = 0, threads = 0, minb = 1;
     std::shared_ptr<BatchKernel> kern;
@@ -661,8 +661,17 @@ extern "C" cufsp_status cufsp_batch_solve(cufsp_batch *B, double t_final, double
             B->gexec = nullptr;
         }
     }
+    // The kernel moves pairs of states, 16 bytes each.  Vectors that start on an 8-byte boundary (a view into
+    // a larger buffer) are solved in an aligned copy: two copies of the vectors beside the solve.
+    double *p = d_packed;
+    const size_t bytes = sizeof(double) * (size_t)B->offsets.back();
+    if (reinterpret_cast<uintptr_t>(d_packed) % 16 != 0) {
+        if (!B->d_scratch) CUFSP_CUDA_TRY(dev_malloc(&B->d_scratch, bytes));
+        p = B->d_scratch;
+        CUFSP_CUDA_TRY(cudaMemcpyAsync(p, d_packed, bytes, cudaMemcpyDeviceToDevice, st));
+    }
     // replay the solve as a CUDA graph (re-captured when the final time, the vectors or the stream change)
-    if (!B->gexec || B->g_tfinal != t_final || B->g_p != d_packed || B->g_stream != st) {
+    if (!B->gexec || B->g_tfinal != t_final || B->g_p != p || B->g_stream != st) {
         if (B->gexec) {
             cudaGraphExecDestroy(B->gexec);
             B->gexec = nullptr;
@@ -673,7 +682,7 @@ extern "C" cufsp_status cufsp_batch_solve(cufsp_batch *B, double t_final, double
         cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
         cufsp_status s = CUFSP_SUCCESS;
         if (e == cudaSuccess)
-            s = launch(B, *B->kern, B->cluster, B->threads, B->n_clusters, t_final, d_packed, B->d_order, B->n_inst, cs);
+            s = launch(B, *B->kern, B->cluster, B->threads, B->n_clusters, t_final, p, B->d_order, B->n_inst, cs);
         cudaError_t e2 = cudaStreamEndCapture(cs, &g);
         cudaStreamDestroy(cs);
         if (e != cudaSuccess || s != CUFSP_SUCCESS || e2 != cudaSuccess) {
@@ -684,10 +693,11 @@ extern "C" cufsp_status cufsp_batch_solve(cufsp_batch *B, double t_final, double
         cudaGraphDestroy(g);
         if (e != cudaSuccess) return cuda_error(e, "cufsp_batch_solve: graph instantiate");
         B->g_tfinal = t_final;
-        B->g_p = d_packed;
+        B->g_p = p;
         B->g_stream = st;
     }
     CUFSP_CUDA_TRY(cudaGraphLaunch(B->gexec, st));
+    if (p != d_packed) CUFSP_CUDA_TRY(cudaMemcpyAsync(d_packed, p, bytes, cudaMemcpyDeviceToDevice, st));
     std::vector<CufspBatchStat> hs(B->n_inst);
     CUFSP_CUDA_TRY(cudaMemcpyAsync(hs.data(), B->d_stats, sizeof(CufspBatchStat) * B->n_inst, cudaMemcpyDeviceToHost, st));
     CUFSP_CUDA_TRY(cudaStreamSynchronize(st));
