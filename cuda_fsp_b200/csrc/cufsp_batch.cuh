@@ -529,7 +529,7 @@ __device__ __noinline__ void pass_dots(Shared &s, const double *v, const double 
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
                 x[k] = make_double2(0.0, 0.0);
-                if (k < used) x[k] = ld2((k ? pn + (k - 1) * ld : p0) + i, two);
+                if (k < used) x[k] = ld2((k ? pn + (size_t)(k - 1) * ld : p0) + i, two);
             }
 #pragma unroll
             for (int k = 0; k < 8; ++k) acc[k] = fma(x[k].y, wi.y, fma(x[k].x, wi.x, acc[k]));
@@ -552,7 +552,7 @@ __device__ __noinline__ double pass_update(const double *v, const double *W, int
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
                 x[k] = make_double2(0.0, 0.0);
-                if (g0 + k < K) x[k] = ld2(k ? pn + (k - 1) * ld : p0, two);
+                if (g0 + k < K) x[k] = ld2(k ? pn + (size_t)(k - 1) * ld : p0, two);
             }
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
@@ -578,7 +578,7 @@ __device__ __noinline__ void pass_combine(double *v, const double *W, int ld, in
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
                 x[k] = make_double2(0.0, 0.0);
-                if (g0 + k < K) x[k] = ld2(k ? pn + (k - 1) * ld : p0, two);
+                if (g0 + k < K) x[k] = ld2(k ? pn + (size_t)(k - 1) * ld : p0, two);
             }
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
