@@ -411,7 +411,9 @@ struct PArnoldi {
     int *d_rterm = nullptr;
     int64_t *d_d = nullptr;
     double *d_props = nullptr;  // sparse formats: exported propensities
+    bool have_model = false;  // the model data above has arrived
     double *d_ex = nullptr;  // two exchange areas: a launch uses one and clears the other
+    bool clean = false;      // so that the next launch's is unset: the last launch has reported
     int ex_rows = 0;         // rows per area
     int turn = 0;            // area of the next launch
     int grid = 0, chunk = 0, slots = 0, ring = 0;
@@ -441,6 +443,8 @@ void parnoldi_destroy(PArnoldi *pa) {
 void parnoldi_destroy(PArnoldi *pa, cudaStream_t last_use) {
     parnoldi_release(pa, [last_use](void *p) { cache_free(p, last_use); });
 }
+
+void parnoldi_reported(PArnoldi *pa) { pa->clean = true; }
 
 void parnoldi_thread_disable(bool off) { tl_disabled = off; }
 
@@ -507,15 +511,16 @@ cufsp_status build_terms(PArnoldi *pa, cufsp_mat *A, const std::vector<double> &
     if (T > kMaxTerms) return set_error(CUFSP_ERR_UNSUPPORTED, "persistent Arnoldi: more than 63 distinct shifts");
     shifts.push_back(0);
     // model data on the device (once per generator), in order on st like the build below
-    if (!pa->d_nu) {
-        CUFSP_CUDA_TRY(cache_alloc((void **)&pa->d_nu, sizeof(int) * (size_t)nr * ns));
+    tm.coefs.clear();  // a build that fails leaves no table behind
+    if (!pa->have_model) {
+        if (!pa->d_nu) CUFSP_CUDA_TRY(cache_alloc((void **)&pa->d_nu, sizeof(int) * (size_t)nr * ns));
         CUFSP_CUDA_TRY(cudaMemcpyAsync(pa->d_nu, m.nu.data(), sizeof(int) * (size_t)nr * ns, cudaMemcpyHostToDevice, st));
-        CUFSP_CUDA_TRY(cache_alloc((void **)&pa->d_c, sizeof(double) * nr));
-        CUFSP_CUDA_TRY(cache_alloc((void **)&pa->d_rterm, sizeof(int) * nr * 2));
-        CUFSP_CUDA_TRY(cache_alloc((void **)&pa->d_d, sizeof(int64_t) * nr));
+        if (!pa->d_c) CUFSP_CUDA_TRY(cache_alloc((void **)&pa->d_c, sizeof(double) * nr));
+        if (!pa->d_rterm) CUFSP_CUDA_TRY(cache_alloc((void **)&pa->d_rterm, sizeof(int) * nr * 2));
+        if (!pa->d_d) CUFSP_CUDA_TRY(cache_alloc((void **)&pa->d_d, sizeof(int64_t) * nr));
         CUFSP_CUDA_TRY(cudaMemcpyAsync(pa->d_d, d.data(), sizeof(int64_t) * nr, cudaMemcpyHostToDevice, st));
         if (A->format == CUFSP_FORMAT_KRONECKER) {
-            CUFSP_CUDA_TRY(cache_alloc((void **)&pa->d_tables, sizeof(double) * m.tables.size()));
+            if (!pa->d_tables) CUFSP_CUDA_TRY(cache_alloc((void **)&pa->d_tables, sizeof(double) * m.tables.size()));
             CUFSP_CUDA_TRY(cudaMemcpyAsync(pa->d_tables, m.tables.data(), sizeof(double) * m.tables.size(),
                                            cudaMemcpyHostToDevice, st));
         }
@@ -559,6 +564,7 @@ cufsp_status build_terms(PArnoldi *pa, cufsp_mat *A, const std::vector<double> &
     CUFSP_CUDA_TRY(cudaGetLastError());
     // the copies above read pageable host memory: finish before `rterm` goes out of scope
     CUFSP_CUDA_TRY(cudaStreamSynchronize(st));
+    pa->have_model = true;
     tm.coefs = coefs;
     tm.transpose = transpose;
     tm.T = T;
@@ -652,7 +658,6 @@ cufsp_status parnoldi_run(PArnoldi **ppa, cufsp_mat *A, const std::vector<double
         pa->ex_rows = rows;
         const size_t bytes = sizeof(double) * 2 * (size_t)exchange_doubles(rows, (int)grid);
         CUFSP_CUDA_TRY(cache_alloc((void **)&pa->d_ex, bytes));
-        CUFSP_CUDA_TRY(cudaMemsetAsync(pa->d_ex, kUnsetByte, bytes, st));
         pa->chunk = (int)chunk;
         pa->grid = (int)grid;
     }
@@ -680,6 +685,11 @@ cufsp_status parnoldi_run(PArnoldi **ppa, cufsp_mat *A, const std::vector<double
     a.btol = btol;
     a.with_avnorm = with_avnorm ? 1 : 0;
     const size_t area = (size_t)exchange_doubles(pa->ex_rows, pa->grid);
+    if (!pa->clean) {  // the first launch, or one after a launch that was refused, captured or broke off
+        CUFSP_CUDA_TRY(cudaMemsetAsync(pa->d_ex, kUnsetByte, sizeof(double) * 2 * area, st));
+        CUFSP_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int), st));
+    }
+    pa->clean = false;  // until this one has reported (parnoldi_reported)
     a.ex = pa->d_ex + (size_t)pa->turn * area;
     a.ex_next = pa->d_ex + (size_t)(1 - pa->turn) * area;
     a.ex_rows = pa->ex_rows;

@@ -240,8 +240,9 @@ cufsp_status mat_apply_transpose(cufsp_mat *A, const double *coefs, double alpha
 
 // Persistent single-launch Arnoldi pass for generators whose Krylov basis stays in L2
 // (cufsp_arnoldi.cu).  Writes the same device state block as the launch sequence of
-// cufsp_krylov.cu; *err (zero before) is set when a bounded wait expired.  With h_state (pinned), the
-// first `words` doubles of the block, which starts at H, are copied there and *h_seq is set to seq.
+// cufsp_krylov.cu; *err is set when a bounded wait expired.  With h_state (pinned), the first `words`
+// doubles of the block, which starts at H, are copied there and *h_seq is set to seq.  A caller that has
+// read the block, with no error, says so by parnoldi_reported.
 struct PArnoldi;
 bool parnoldi_wanted(const cufsp_mat *A, int64_t n, int m);
 bool parnoldi_size_ok(int64_t n);  // the size rule of parnoldi_wanted alone
@@ -249,6 +250,7 @@ cufsp_status parnoldi_run(PArnoldi **pa, cufsp_mat *A, const std::vector<double>
                           int64_t n, const double *v, double *W, double *H, double *rho, double *gam, double *beta,
                           double *avnorm, int *flag, int *err, int m, int iop, int q, double btol, bool with_avnorm,
                           double *h_state, int words, unsigned *h_seq, unsigned seq, cudaStream_t st);
+void parnoldi_reported(PArnoldi *pa);
 void parnoldi_destroy(PArnoldi *pa);
 void parnoldi_destroy(PArnoldi *pa, cudaStream_t last_use);  // every launch of pa was ordered on last_use
 // Host threads that run many solves concurrently keep the launch sequence: the persistent pass

@@ -707,13 +707,9 @@ cufsp_status arnoldi_pass(cufsp_expv *E, double *v, cudaStream_t st, bool with_a
     int flag, barrier_err;
     std::memcpy(&flag, hrho + 2 * mp2 + 4, sizeof(int));
     std::memcpy(&barrier_err, reinterpret_cast<const char *>(hrho + 2 * mp2 + 4) + sizeof(int), sizeof(int));
-    if (persistent && barrier_err) {
-        // the exchange rows of the broken-off launch are in no known state: the next pass starts afresh
-        cudaMemsetAsync(E->ks.flag + 1, 0, sizeof(int), st);
-        parnoldi_destroy(E->pa, st);
-        E->pa = nullptr;
-        return set_error(CUFSP_ERR_CUDA, "expv: a grid barrier wait of the persistent Arnoldi pass expired");
-    }
+    if (persistent && barrier_err)
+        return set_error(CUFSP_ERR_CUDA, "expv: a wait between the CTAs of the persistent Arnoldi pass expired");
+    if (persistent) parnoldi_reported(E->pa);
     if (!persistent && E->A) {
         s = mat_check_watchdog(E->A, "expv");
         if (s != CUFSP_SUCCESS) return s;
