@@ -148,6 +148,7 @@ SIGNATURES = {
     "cufsp_bdf_set_coefs": [_P, _DP],
     "cufsp_bdf_init": [_P, C.c_double, _P, _P],
     "cufsp_bdf_advance": [_P, C.c_double, _P, C.c_int, _P, _DP],
+    "cufsp_bdf_describe": [_P, C.c_char_p, C.c_size_t],
     "cufsp_bdf_get_stats": [_P, C.POINTER(BdfStats)],
     "cufsp_solver_create": [_P, _DP, C.c_int, C.c_double, _DP, C.c_double, C.c_int, C.c_int, C.c_int, C.POINTER(_P)],
     "cufsp_solver_create_bdf": [_P, _DP, C.c_int, C.c_double, _DP, C.c_double, C.c_double, C.POINTER(_P)],

@@ -419,8 +419,8 @@ cufsp_status step(cufsp_bdf *B, double t_out, cudaStream_t st) {
     const double eps = 2.220446049250313e-16;
     const double hmax = B->h_max > 0.0 ? B->h_max : INFINITY;
     if (!B->stepper_asked) {
+        BDF_TRY(bdf_stepper_create(B->A, B->maxl, st, &B->stepper));
         B->stepper_asked = true;
-        B->stepper = bdf_stepper_create(B->A, B->maxl, st);
     }
     for (;;) {
         if (B->h > hmax) {
@@ -661,6 +661,16 @@ extern "C" cufsp_status cufsp_bdf_advance(cufsp_bdf *B, double t_out, double *d_
     CUFSP_CUDA_TRY(cudaMemcpyAsync(d_p, B->D[0], sizeof(double) * B->n, cudaMemcpyDeviceToDevice, st));
     CUFSP_CUDA_TRY(cudaStreamSynchronize(st));
     if (t_reached) *t_reached = B->t;
+    return CUFSP_SUCCESS;
+}
+
+extern "C" cufsp_status cufsp_bdf_describe(const cufsp_bdf *B, char *buf, size_t len) {
+    if (!B || !buf || len == 0) return set_error(CUFSP_ERR_INVALID_ARG, "cufsp_bdf_describe: bad argument");
+    const std::string d = "BDF: " + (B->stepper ? bdf_stepper_describe(B->stepper)
+                                                : std::string(B->stepper_asked ? "launch sequence" : "no step taken yet"));
+    const size_t k = std::min(len - 1, d.size());
+    std::memcpy(buf, d.data(), k);
+    buf[k] = 0;
     return CUFSP_SUCCESS;
 }
 

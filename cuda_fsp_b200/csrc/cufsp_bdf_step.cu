@@ -603,7 +603,7 @@ cudaError_t step_smem_attribute() {  // once per device, for every variant (as i
 
 struct BdfStepper {
     StepArgs a;
-    StepKernel kern = nullptr;
+    const StepVariant *var = nullptr;
     int grid = 0;
     size_t smem = 0;
     double *d_units = nullptr;  // gain and outflow tables, then the base table
@@ -628,7 +628,17 @@ void bdf_stepper_destroy(BdfStepper *B) {
     delete B;
 }
 
-BdfStepper *bdf_stepper_create(cufsp_mat *A, int maxl, cudaStream_t st) {
+std::string bdf_stepper_describe(const BdfStepper *B) {
+    const StepArgs &a = B->a;
+    return "one persistent launch per step attempt, " + std::to_string(B->grid) + " CTAs x " + std::to_string(kThreads + 32) +
+           " threads, variant of " + std::to_string(B->var->states / kThreads) + " states per thread, " +
+           std::to_string(B->var->near) + " near and " + std::to_string(B->var->far) + " far terms, " + std::to_string(a.slots) +
+           " of " + std::to_string(a.maxl + 1) + " basis vectors in shared memory, " + std::to_string(a.n_var) +
+           " rates added per launch";
+}
+
+cufsp_status bdf_stepper_create(cufsp_mat *A, int maxl, cudaStream_t st, BdfStepper **out) {
+    *out = nullptr;
     static const bool on = [] {
         const char *e = getenv("CUFSP_BDF_PERSISTENT");
         return !e || atoi(e) != 0;
@@ -639,7 +649,7 @@ BdfStepper *bdf_stepper_create(cufsp_mat *A, int maxl, cudaStream_t st) {
     const int sms = std::min(device_info().sm_count, 64 * kMaxGridPairs);
     const bool kron = A->format == CUFSP_FORMAT_KRONECKER;
     if (!on || nr > kMaxR || maxl > kMaxL || n > (int64_t)sms * kVariants[8].states || (kron ? m.tables.empty() : !A->sparse))
-        return nullptr;
+        return CUFSP_SUCCESS;
     std::vector<int64_t> d(nr, 0), stride(ns, 1);
     for (int s = 1; s < ns; ++s) stride[s] = stride[s - 1] * ((int64_t)m.bounds[s - 1] + 1);
     for (int r = 0; r < nr; ++r)
@@ -662,9 +672,9 @@ BdfStepper *bdf_stepper_create(cufsp_mat *A, int maxl, cudaStream_t st) {
         if (!var && a.chunk <= v.states && a.terms.n_near <= v.near && a.terms.n_far <= v.far) var = &v;
     if (!var) {
         delete B;
-        return nullptr;
+        return CUFSP_SUCCESS;
     }
-    B->kern = var->kern;
+    B->var = var;
     a.nr = nr;
     for (int r = 0; r < nr; ++r) {
         a.term[r] = -1;
@@ -702,8 +712,9 @@ BdfStepper *bdf_stepper_create(cufsp_mat *A, int maxl, cudaStream_t st) {
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_nu, m.nu.data(), sizeof(int) * (size_t)nr * ns, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_d, d.data(), sizeof(int64_t) * nr, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess && kron) e = cudaMemcpyAsync(d_tab, m.tables.data(), sizeof(double) * tab, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess && !kron && sparse_export(A->sparse, d_tab, st) != CUFSP_SUCCESS) e = cudaErrorUnknown;
-    if (e == cudaSuccess) {
+    cufsp_status s = CUFSP_SUCCESS;
+    if (e == cudaSuccess && !kron) s = sparse_export(A->sparse, d_tab, st);
+    if (e == cudaSuccess && s == CUFSP_SUCCESS) {
         UnitArgs u;
         std::memset(&u, 0, sizeof(u));
         u.n = n;
@@ -729,11 +740,12 @@ BdfStepper *bdf_stepper_create(cufsp_mat *A, int maxl, cudaStream_t st) {
     cache_free(d_d, st);
     int per_sm = 0;
     if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)B->kern, kThreads + 32, B->smem);
-    if (e != cudaSuccess || per_sm < 1) {
-        cudaGetLastError();
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)var->kern, kThreads + 32, B->smem);
+    if (e != cudaSuccess || s != CUFSP_SUCCESS || per_sm < 1) {
         bdf_stepper_destroy(B);
-        return nullptr;
+        if (e != cudaSuccess && e != cudaErrorMemoryAllocation) return cuda_error(e, "cufsp_bdf: persistent step");
+        cudaGetLastError();
+        return s;
     }
     a.gain = B->d_units;
     a.out = B->d_units + units;
@@ -741,7 +753,8 @@ BdfStepper *bdf_stepper_create(cufsp_mat *A, int maxl, cudaStream_t st) {
     a.err = B->d_err;
     B->used = true;  // the unit tables were built on st
     B->last = st;
-    return B;
+    *out = B;
+    return CUFSP_SUCCESS;
 }
 
 cufsp_status bdf_stepper_run(BdfStepper *B, const BdfStepIn &in, BdfStepOut &out, cudaStream_t st) {
@@ -804,7 +817,7 @@ cufsp_status bdf_stepper_run(BdfStepper *B, const BdfStepIn &in, BdfStepOut &out
     if (B->last != st) B->mixed = true;
     B->last = st;
     void *args[] = {&a};
-    CUFSP_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)B->kern, dim3(B->grid), dim3(kThreads + 32), args, B->smem, st));
+    CUFSP_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)B->var->kern, dim3(B->grid), dim3(kThreads + 32), args, B->smem, st));
     // bounded poll of the report, as the integrator's scalar reads
     const auto t0 = std::chrono::steady_clock::now();
     const volatile unsigned *seq = a.h_seq;

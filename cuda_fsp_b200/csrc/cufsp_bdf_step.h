@@ -32,9 +32,11 @@ struct BdfStepOut {
     double em, ep;       // ||D_k||_w, ||D_{k+2}||_w after an accepted step
 };
 
-// The stepper for a generator, or nullptr when the launch sequence is to be used (size or network out
-// of range, CUFSP_BDF_PERSISTENT=0, or memory short).
-BdfStepper *bdf_stepper_create(cufsp_mat *A, int maxl, cudaStream_t st);
+// The stepper for a generator; *out = nullptr when the launch sequence is to be used (size or network out
+// of range, CUFSP_BDF_PERSISTENT=0, or memory short).  Any other failure is an error, and the caller may ask
+// again.
+cufsp_status bdf_stepper_create(cufsp_mat *A, int maxl, cudaStream_t st, BdfStepper **out);
+std::string bdf_stepper_describe(const BdfStepper *B);
 void bdf_stepper_destroy(BdfStepper *B);
 cufsp_status bdf_stepper_run(BdfStepper *B, const BdfStepIn &in, BdfStepOut &out, cudaStream_t st);
 

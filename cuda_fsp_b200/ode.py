@@ -64,6 +64,11 @@ class BDFIntegrator:
         _lib.check(self._lib, self._lib.cufsp_bdf_get_stats(self._h, C.byref(st)), "cufsp_bdf_get_stats")
         return st.as_dict()
 
+    def describe(self) -> str:
+        buf = C.create_string_buffer(512)
+        _lib.check(self._lib, self._lib.cufsp_bdf_describe(self._h, buf, len(buf)), "cufsp_bdf_describe")
+        return buf.value.decode()
+
     def close(self) -> None:
         if getattr(self, "_h", None) and self._h.value:
             self._lib.cufsp_bdf_destroy(self._h)

@@ -222,6 +222,9 @@ cufsp_status cufsp_bdf_set_coefs(cufsp_bdf *B, const double *coefs);
 cufsp_status cufsp_bdf_init(cufsp_bdf *B, double t0, const double *d_p0, cufsp_stream_t stream);
 cufsp_status cufsp_bdf_advance(cufsp_bdf *B, double t_out, double *d_p, int one_step, cufsp_stream_t stream,
                                double *t_reached);
+/* How the steps are taken (one persistent launch per attempt, and in which variant, or a launch sequence),
+   as text. */
+cufsp_status cufsp_bdf_describe(const cufsp_bdf *B, char *buf, size_t len);
 cufsp_status cufsp_bdf_get_stats(const cufsp_bdf *B, cufsp_bdf_stats *stats);
 
 /* ---- FSP solver through output times ------------------------------------------------------

@@ -1,0 +1,42 @@
+"""Which form of the BDF step a generator gets (gpu, 148 SMs): the variant of the persistent launch by states per
+CTA and by terms, the basis vectors its shared memory holds, and the launch sequence where none applies."""
+import re
+
+import pytest
+
+from cuda_fsp_b200 import BDFIntegrator, FSPMat, MatrixFormat, models
+
+pytestmark = pytest.mark.gpu
+
+# states per thread, near and far terms of the variant, whether the whole basis is in shared memory
+FORMS = {
+    "one_state": (lambda: models.toggle((210, 200), time_varying=True), "KRONECKER", 30, (1, 4, 2, True)),
+    "one_state_many_far": (lambda: models.mass_action_3(bounds=(70, 20, 20)), "KRONECKER", 30, (1, 4, 8, True)),
+    "two_states_many_near": (lambda: models.gene_expression((1, 1, 1, 90, 100)), "KRONECKER", 30, (2, 10, 4, True)),
+    "three_states_many_far": (lambda: models.mass_action_3(bounds=(70, 50, 30)), "KRONECKER", 30, (3, 4, 8, True)),
+    "one_cta": (lambda: models.toggle((12, 9), time_varying=True), "KRONECKER", 30, (1, 10, 4, True)),
+    "hyb": (lambda: models.gene_expression((1, 1, 1, 40, 30)), "HYB", 30, (1, 10, 4, True)),
+    "basis_partly_in_l2": (lambda: models.mass_action_3(bounds=(70, 50, 40)), "KRONECKER", 60, (3, 4, 8, False)),
+    "too_many_states": (lambda: models.mass_action_3(bounds=(70, 50, 43)), "KRONECKER", 30, None),
+}
+
+
+@pytest.mark.parametrize("name", FORMS)
+def test_form_of_the_step(cuda, name, monkeypatch):
+    import torch
+    make, fmt, maxl, want = FORMS[name]
+    m = make()
+    B = BDFIntegrator(FSPMat.from_model(m, getattr(MatrixFormat, fmt)), rtol=1e-6, atol=1e-12, maxl=maxl)
+    assert B.describe() == "BDF: no step taken yet"
+    p = torch.as_tensor(m.p0(), device="cuda")
+    B.init(0.0, p)
+    B.step(1e-3, p)
+    d = B.describe()
+    if want is None:
+        assert d == "BDF: launch sequence"
+        return
+    got = re.search(r"persistent launch .* variant of (\d) states per thread, (\d+) near and (\d+) far terms, (\d+) of (\d+) basis", d)
+    assert got, d
+    s, near, far, slots, vecs = (int(v) for v in got.groups())
+    assert (s, near, far, slots == vecs) == want, d
+    assert vecs == maxl + 1
