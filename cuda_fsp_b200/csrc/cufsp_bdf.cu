@@ -605,6 +605,7 @@ extern "C" cufsp_status cufsp_bdf_set_coefs(cufsp_bdf *B, const double *coefs) {
         return set_error(CUFSP_ERR_INVALID_ARG, "cufsp_bdf_set_coefs: no coefficients and the generator has no tcoef");
     B->fixed = coefs != nullptr;
     if (coefs) B->coefs.assign(coefs, coefs + B->A->model.nr);
+    if (B->stepper) bdf_stepper_new_rates(B->stepper);
     B->ready = false;
     return CUFSP_SUCCESS;
 }

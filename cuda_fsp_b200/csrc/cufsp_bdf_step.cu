@@ -619,6 +619,11 @@ struct BdfStepper {
     bool fresh = false;         // both sets are unset
 };
 
+void bdf_stepper_new_rates(BdfStepper *B) {
+    B->have_base = false;
+    B->varying = 0;
+}
+
 void bdf_stepper_destroy(BdfStepper *B) {
     if (!B) return;
     for (void *p : {(void *)B->d_units, (void *)B->d_X, (void *)B->d_ex, (void *)B->d_err}) {

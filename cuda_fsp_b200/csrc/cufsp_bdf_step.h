@@ -37,6 +37,7 @@ struct BdfStepOut {
 // again.
 cufsp_status bdf_stepper_create(cufsp_mat *A, int maxl, cudaStream_t st, BdfStepper **out);
 std::string bdf_stepper_describe(const BdfStepper *B);
+void bdf_stepper_new_rates(BdfStepper *B);  // the rates to come are others: none has varied yet
 void bdf_stepper_destroy(BdfStepper *B);
 cufsp_status bdf_stepper_run(BdfStepper *B, const BdfStepIn &in, BdfStepOut &out, cudaStream_t st);
 

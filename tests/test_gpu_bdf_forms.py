@@ -40,3 +40,37 @@ def test_form_of_the_step(cuda, name, monkeypatch):
     s, near, far, slots, vecs = (int(v) for v in got.groups())
     assert (s, near, far, slots == vecs) == want, d
     assert vecs == maxl + 1
+
+
+def test_new_rates_are_not_varying_rates(cuda):
+    """After set_coefs no rate is added launch by launch, and the steps are those of a new integrator."""
+    import numpy as np
+    import torch
+    m = models.gene_expression((1, 1, 1, 30, 40), time_varying=False)
+    A = FSPMat.from_model(m, MatrixFormat.KRONECKER)
+    c = m.coefs(0) * np.linspace(0.8, 1.2, m.nr)
+    p0 = torch.as_tensor(m.p0(), device="cuda")
+    out = []
+    for first in (m.coefs(0), c):
+        B = BDFIntegrator(A, coefs=first, rtol=1e-8, atol=1e-14)
+        p = p0.clone()
+        if first is not c:
+            B.init(0.0, p0)
+            B.advance(0.5, p)
+            B.set_coefs(c)
+        B.init(0.0, p0)
+        B.advance(1.0, p)
+        assert " 0 rates added" in B.describe()
+        out.append((p.cpu().numpy(), B.stats))
+    assert out[0][1] == out[1][1]
+    assert np.array_equal(out[0][0], out[1][0])
+
+
+def test_varying_rates_are_counted(cuda):
+    import torch
+    m = models.gene_expression((1, 1, 1, 30, 40))  # one switching rate
+    B = BDFIntegrator(FSPMat.from_model(m, MatrixFormat.KRONECKER), rtol=1e-6, atol=1e-12)
+    p = torch.as_tensor(m.p0(), device="cuda")
+    B.init(0.0, p)
+    B.advance(1.0, p)
+    assert " 1 rates added" in B.describe()
