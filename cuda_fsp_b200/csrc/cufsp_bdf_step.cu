@@ -609,7 +609,7 @@ struct BdfStepper {
     double *d_units = nullptr;  // gain and outflow tables, then the base table
     double base_coef[kMaxR];    // rates in the base table
     unsigned varying = 0;       // reactions left out of it: their rates have changed before
-    bool have_base = false;
+    bool have_base = false;     // (the launch that followed its build has reported)
     double *d_X = nullptr;      // two sets of published vectors: a launch uses one and clears the other
     double *d_ex = nullptr;     // two exchange areas, likewise
     int *d_err = nullptr;
@@ -770,6 +770,8 @@ cufsp_status bdf_stepper_run(BdfStepper *B, const BdfStepIn &in, BdfStepOut &out
         CUFSP_CUDA_TRY(cudaMemsetAsync(B->d_ex, kUnsetByte, sizeof(double) * 2 * area, st));
         CUFSP_CUDA_TRY(cudaMemsetAsync(B->d_err, 0, sizeof(int), st));
         B->used_vecs = B->used_rows = 0;
+        B->have_base = false;  // nor is the base table known to have been built
+        B->varying = 0;
     }
     B->fresh = false;  // until the launch has reported
     for (int j = 0; j < kBdfHist; ++j) a.D[j] = in.D[j];

@@ -6,7 +6,7 @@ from contextlib import contextmanager
 import numpy as np
 import pytest
 
-from cuda_fsp_b200 import CufspError, FSPMat, KryExpvFSP, MatrixFormat, models
+from cuda_fsp_b200 import BDFIntegrator, CufspError, FSPMat, KryExpvFSP, MatrixFormat, models
 
 pytestmark = pytest.mark.gpu
 
@@ -45,4 +45,36 @@ def test_krylov_solve_after_a_captured_step(cuda, fmt, steps_before):
         stats.append(E.solve(stream=s.cuda_stream))
         out.append(v.cpu().numpy())
     assert stats[0] == stats[1] and stats[0]["n_steps"] > steps_before
+    assert np.array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("steps_before", [0, 1, 4])
+def test_bdf_after_a_captured_step(cuda, steps_before):
+    """The captured attempt is the first with new rates, so that it has rebuilt the coefficient table (given an
+    initial step, the start of an integration waits for nothing)."""
+    import torch
+    m = models.toggle((50, 41))
+    c = m.coefs(0) * np.linspace(0.7, 1.3, m.nr)
+    s = torch.cuda.Stream()
+    out, stats = [], []
+    for capture in (False, True):
+        A = FSPMat.from_model(m, MatrixFormat.HYB)
+        p0 = torch.as_tensor(m.p0(), device="cuda")
+        p = p0.clone()
+        torch.cuda.synchronize()
+        B = BDFIntegrator(A, coefs=m.coefs(0), rtol=1e-8, atol=1e-14, h_init=1e-3)
+        B.init(0.0, p0, stream=s.cuda_stream)
+        for _ in range(steps_before):
+            B.step(50.0, p, stream=s.cuda_stream)
+        B.set_coefs(c)
+        if capture:
+            with capturing(s):
+                B.init(0.0, p0, stream=s.cuda_stream)
+                with pytest.raises(CufspError):
+                    B.advance(50.0, p, stream=s.cuda_stream)
+        B.init(0.0, p0, stream=s.cuda_stream)
+        B.advance(50.0, p, stream=s.cuda_stream)
+        stats.append(B.stats)
+        out.append(p.cpu().numpy())
+    assert stats[0] == stats[1]
     assert np.array_equal(out[0], out[1])
