@@ -513,17 +513,20 @@ extern "C" cufsp_status cufsp_likelihood_grad_batched(const cufsp_model_desc *de
     // passes of two workers in turn (one's host work beside the other's pass).  Gradients/s of 16 sets, 4 workers
     // asked for, shares and turns: 64,800 states 5.97 and 5.11, 93,312 states (630 per SM) 4.36 and 4.21,
     // 131,072 states (886 per SM) 2.55 and 3.11.
-    // CUFSP_GRAD_SM_SHARE=0 or 1: always turns, always shares.  Larger generators run `workers` concurrent
-    // launch sequences.
+    // Turns, too, where a share's two working slices would not fit its shared memory (14,256 states per CTA:
+    // 32 workers have 4 CTAs each, enough for 57,024 states).
+    // CUFSP_GRAD_SM_SHARE=0 or 1: always turns, shares wherever they fit.  Larger generators run `workers`
+    // concurrent launch sequences.
     constexpr int64_t kShareStates = 700;
     int64_t n_states = 1;
     for (int s = 0; s < desc->n_species; ++s) n_states *= (int64_t)desc->fsp_bounds[s] + 1;
-    const bool persistent = parnoldi_size_ok(n_states);
     const int sms = device_info().sm_count;
+    const bool persistent = parnoldi_size_ok(n_states) && parnoldi_fits(n_states, sms);
     const char *share_env = getenv("CUFSP_GRAD_SM_SHARE");
-    const bool share = share_env ? atoi(share_env) != 0 : n_states <= kShareStates * sms;
+    const int part = std::max(1, sms / workers);
+    const bool share = (share_env ? atoi(share_env) != 0 : n_states <= kShareStates * sms) && parnoldi_fits(n_states, part);
     int cta_cap = 0;
-    if (persistent && share) cta_cap = std::max(1, sms / workers);
+    if (persistent && share) cta_cap = part;
     else if (persistent) workers = std::min(workers, 2);
     int dev = 0;
     CUFSP_CUDA_TRY(cudaGetDevice(&dev));

@@ -472,8 +472,36 @@ bool parnoldi_size_ok(int64_t n) {
     return mode != 0 && (mode == 1 || n <= max_n);
 }
 
+namespace {
+// Dynamic shared memory the pass may use, and what it needs beside the basis: the CTA's slices of W_j and
+// A W_j, and W_j's halo.
+size_t persistent_smem_max() { return (size_t)device_info().max_smem_optin - sizeof(PSmem) - 1024; }
+size_t persistent_fixed(int64_t chunk) { return sizeof(double) * (2 * (size_t)chunk + 2 * kHaloMax); }
+
+// States per CTA (even) of a pass that may use `ctas` CTAs: one CTA per SM, fewer for small n, each with at
+// least 256 states by default (CUFSP_ARNOLDI_CTA_STATES).
+int64_t persistent_chunk(int64_t n, int ctas) {
+    static const int64_t min_states = [] {
+        const char *e = getenv("CUFSP_ARNOLDI_CTA_STATES");
+        return e ? std::max<int64_t>(32, atoll(e)) : (int64_t)256;
+    }();
+    const int64_t want = std::max<int64_t>(1, std::min<int64_t>(ctas, (n + min_states - 1) / min_states));
+    return ((n + want - 1) / want + 1) & ~int64_t(1);
+}
+
+// CTAs a pass launched from this thread may use.
+int persistent_ctas() {
+    const int sms = std::min(device_info().sm_count, 64 * kMaxGridPairs);
+    return tl_cta_cap > 0 ? std::min(tl_cta_cap, sms) : sms;
+}
+}  // namespace
+
+bool parnoldi_fits(int64_t n, int ctas) {
+    return n <= INT32_MAX / 2 && persistent_fixed(persistent_chunk(n, ctas)) <= persistent_smem_max();
+}
+
 bool parnoldi_wanted(const cufsp_mat *A, int64_t n, int m) {
-    if (tl_disabled || !A || m > CUFSP_MAX_KRYLOV || !parnoldi_size_ok(n)) return false;
+    if (tl_disabled || !A || m > CUFSP_MAX_KRYLOV || !parnoldi_size_ok(n) || !parnoldi_fits(n, persistent_ctas())) return false;
     if (A->model.nr > CUFSP_MAX_REACTIONS_SPARSE || A->model.ns > CUFSP_MAX_SPECIES) return false;
     return A->format == CUFSP_FORMAT_KRONECKER ? !A->model.tables.empty() : A->sparse != nullptr;
 }
@@ -587,9 +615,6 @@ const PVariant kPVariants[] = {CUFSP_PV(1, 4, 2), CUFSP_PV(1, 10, 4), CUFSP_PV(1
                                {k_arnoldi_persistent<512, 1, 0, 0>, 512, INT32_MAX, kMaxTerms, kMaxTerms}};
 #undef CUFSP_PV
 
-// Dynamic shared memory the pass may use.
-size_t persistent_smem_max() { return (size_t)device_info().max_smem_optin - sizeof(PSmem) - 1024; }
-
 cudaError_t persistent_smem_attribute() {
     constexpr int kMaxDevices = 64;
     static std::mutex mu;
@@ -621,24 +646,15 @@ cufsp_status parnoldi_run(PArnoldi **ppa, cufsp_mat *A, const std::vector<double
     cufsp_status s = build_terms(pa, A, coefs, transpose, tm, st);
     if (s != CUFSP_SUCCESS) return s;
     if (!pa->grid) {
-        // One CTA per SM (fewer for small n: at least 256 states each by default); the CTA's slice
-        // of the newest vector must fit its shared memory.
-        static const int64_t min_states = [] {  // states per CTA at least (CUFSP_ARNOLDI_CTA_STATES)
-            const char *e = getenv("CUFSP_ARNOLDI_CTA_STATES");
-            return e ? std::max<int64_t>(32, atoll(e)) : (int64_t)256;
-        }();
         // a host thread that shares the GPU with other solves (the batched gradient's workers) takes
         // its share of the SMs, so that the workers' cooperative passes run side by side
-        const int sms = std::min(device_info().sm_count, 64 * kMaxGridPairs);
-        const int cap = tl_cta_cap > 0 ? std::min(tl_cta_cap, sms) : sms;
-        const int64_t want = std::max<int64_t>(1, std::min<int64_t>(cap, (n + min_states - 1) / min_states));
-        const int64_t chunk = ((n + want - 1) / want + 1) & ~int64_t(1);
+        const int64_t chunk = persistent_chunk(n, persistent_ctas());
         const int64_t grid = (n + chunk - 1) / chunk;
         const size_t row = sizeof(double) * (size_t)chunk, room = persistent_smem_max();
         if (n > INT32_MAX / 2) return set_error(CUFSP_ERR_UNSUPPORTED, "persistent Arnoldi: too many states");
         // basis vectors the dots read: W_0..W_{m-1}, or the last q of them
         const bool window = iop && q < m;
-        const size_t fixed = 2 * row + 2 * kHaloMax * sizeof(double);
+        const size_t fixed = persistent_fixed(chunk);
         if (fixed > room) return set_error(CUFSP_ERR_UNSUPPORTED, "persistent Arnoldi: vector slice exceeds shared memory");
         pa->slots = (int)std::min<size_t>((size_t)(window ? q : m), (room - fixed) / row);
         pa->ring = window && pa->slots == q ? q : 0;

@@ -246,6 +246,7 @@ cufsp_status mat_apply_transpose(cufsp_mat *A, const double *coefs, double alpha
 struct PArnoldi;
 bool parnoldi_wanted(const cufsp_mat *A, int64_t n, int m);
 bool parnoldi_size_ok(int64_t n);  // the size rule of parnoldi_wanted alone
+bool parnoldi_fits(int64_t n, int ctas);  // the slices of n states fit the shared memory of `ctas` CTAs
 cufsp_status parnoldi_run(PArnoldi **pa, cufsp_mat *A, const std::vector<double> &coefs, bool transpose,
                           int64_t n, const double *v, double *W, double *H, double *rho, double *gam, double *beta,
                           double *avnorm, int *flag, int *err, int m, int iop, int q, double btol, bool with_avnorm,
