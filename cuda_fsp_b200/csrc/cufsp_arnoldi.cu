@@ -349,7 +349,7 @@ struct TermBuildArgs {
     const double *props;   // [nr][n] propensities a_r(x_i), or null
     const int *nu;         // [nr][ns]
     const double *c;       // [nr] coefficients
-    const int *rterm;      // [nr] term of reaction r (-1: no net change)
+    const int *rterm;      // [nr] term of reaction r (-1: no source inside the box, -2: no net change)
     const int64_t *d;      // [nr] flat shift sum_s nu_{r,s} stride_s
     double *coef;          // [T][n]
 };
@@ -374,10 +374,11 @@ __global__ void k_build_terms(const TermBuildArgs b) {
         double acc[kMaxTerms];
         for (int t = 0; t < b.T; ++t) acc[t] = 0.0;
         for (int r = 0; r < b.nr; ++r) {
+            const int t = b.rterm[r];
+            if (t == -2) continue;  // its gain and its outflow cancel
             const double cr = b.c[r];
             const double here = prop_at(b, r, i, xs);
             acc[b.T - 1] -= cr * here;  // the diagonal keeps the full outflow
-            const int t = b.rterm[r];
             if (t < 0) continue;
             const int sg = b.transpose ? 1 : -1;  // A: source x - nu_r;  A^T: target x + nu_r
             bool ok = true;
@@ -526,7 +527,11 @@ cufsp_status build_terms(PArnoldi *pa, cufsp_mat *A, const std::vector<double> &
     std::vector<int> rterm(nr, -1);
     std::vector<int64_t> shifts;
     for (int r = 0; r < nr; ++r) {
-        if (d[r] == 0) continue;
+        if (d[r] == 0) {  // a change of several species may make up a flat shift of 0, but never inside the box
+            const int *nu = m.nu.data() + (size_t)r * ns;
+            if (std::all_of(nu, nu + ns, [](int v) { return v == 0; })) rterm[r] = -2;
+            continue;
+        }
         const int64_t sh = transpose ? -d[r] : d[r];
         auto it = idx.find(sh);
         if (it == idx.end()) {
