@@ -399,7 +399,8 @@ cufsp_status attempt(cufsp_bdf *B, double t_new, double c, cudaStream_t st, int 
     in.h_out = B->h_scal;
     in.h_seq = B->h_seq;
     in.seq = &B->seq;
-    static_assert(kBdfOutWords <= kNScal, "report block");
+    in.d_out = spin_fetch() ? nullptr : B->d_scal;
+    static_assert(kBdfOutWords + 1 <= kNScal, "report block");
     BdfStepOut out;
     BDF_TRY(bdf_stepper_run(B->stepper, in, out, st));
     B->st.n_matvec += 1 + out.iters;

@@ -65,7 +65,7 @@ struct StepArgs {
     int rows_clear;
     double *ex, *ex_clear;
     int ex_rows;
-    double *h_out;                    // pinned host block and its sequence word
+    double *h_out;                    // report block (pinned host or device memory) and its sequence word
     unsigned *h_seq, seq;
     int *err;
 };
@@ -617,6 +617,7 @@ struct BdfStepper {
     cudaStream_t last = nullptr;  // stream of the launches, unless they were on several (mixed)
     bool used = false, mixed = false;
     bool fresh = false;         // both sets are unset
+    bool copied = false;        // the last report was copied, not polled
 };
 
 void bdf_stepper_new_rates(BdfStepper *B) {
@@ -639,7 +640,7 @@ std::string bdf_stepper_describe(const BdfStepper *B) {
            " threads, variant of " + std::to_string(B->var->states / kThreads) + " states per thread, " +
            std::to_string(B->var->near) + " near and " + std::to_string(B->var->far) + " far terms, " + std::to_string(a.slots) +
            " of " + std::to_string(a.maxl + 1) + " basis vectors in shared memory, " + std::to_string(a.n_var) +
-           " rates added per launch";
+           " rates added per launch, report " + (B->copied ? "copied" : "polled");
 }
 
 cufsp_status bdf_stepper_create(cufsp_mat *A, int maxl, cudaStream_t st, BdfStepper **out) {
@@ -769,6 +770,7 @@ cufsp_status bdf_stepper_run(BdfStepper *B, const BdfStepIn &in, BdfStepOut &out
         CUFSP_CUDA_TRY(cudaMemsetAsync(B->d_X, kUnsetByte, sizeof(double) * 2 * xset, st));
         CUFSP_CUDA_TRY(cudaMemsetAsync(B->d_ex, kUnsetByte, sizeof(double) * 2 * area, st));
         CUFSP_CUDA_TRY(cudaMemsetAsync(B->d_err, 0, sizeof(int), st));
+        if (in.d_out) CUFSP_CUDA_TRY(cudaMemsetAsync(in.d_out, 0, sizeof(double) * (kBdfOutWords + 1), st));
         B->used_vecs = B->used_rows = 0;
         B->have_base = false;  // nor is the base table known to have been built
         B->varying = 0;
@@ -818,16 +820,22 @@ cufsp_status bdf_stepper_run(BdfStepper *B, const BdfStepIn &in, BdfStepOut &out
     a.ex_clear = B->d_ex + (size_t)(1 - B->turn) * area;
     a.n_clear = B->used_vecs;
     a.rows_clear = B->used_rows;
-    a.h_out = in.h_out;
-    a.h_seq = in.h_seq;
+    a.h_out = in.d_out ? in.d_out : in.h_out;
+    a.h_seq = in.d_out ? reinterpret_cast<unsigned *>(in.d_out + kBdfOutWords) : in.h_seq;
     a.seq = ++*in.seq;
+    B->copied = in.d_out != nullptr;
     if (B->last != st) B->mixed = true;
     B->last = st;
     void *args[] = {&a};
     CUFSP_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)B->var->kern, dim3(B->grid), dim3(kThreads + 32), args, B->smem, st));
+    const volatile unsigned *seq = in.h_seq;
+    if (in.d_out) {
+        CUFSP_CUDA_TRY(cudaMemcpyAsync(in.h_out, in.d_out, sizeof(double) * (kBdfOutWords + 1), cudaMemcpyDeviceToHost, st));
+        CUFSP_CUDA_TRY(cudaStreamSynchronize(st));
+        seq = reinterpret_cast<unsigned *>(in.h_out + kBdfOutWords);
+    }
     // bounded poll of the report, as the integrator's scalar reads
     const auto t0 = std::chrono::steady_clock::now();
-    const volatile unsigned *seq = a.h_seq;
     for (unsigned it = 1; *seq != a.seq; ++it) {
         if ((it & 1023) == 0) {
             if (cudaStreamQuery(st) != cudaErrorNotReady) break;

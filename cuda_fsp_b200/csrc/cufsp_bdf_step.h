@@ -19,8 +19,9 @@ struct BdfStepIn {
     double econst;          // error constant of order k
     double atol, rtol, sqrt_n, eps_lin;
     const double *coefs;    // host: c_r(t_new)
-    double *h_out;          // pinned host block of kBdfOutWords doubles, the sequence word that says when it
+    double *h_out;          // pinned host block of kBdfOutWords + 1 doubles, the sequence word that says when it
     unsigned *h_seq, *seq;  // has been written, and its counter
+    double *d_out;          // not null: the launch reports into this device block, which is copied to h_out
 };
 constexpr int kBdfOutWords = 8;
 

@@ -74,3 +74,30 @@ def test_varying_rates_are_counted(cuda):
     B.init(0.0, p)
     B.advance(1.0, p)
     assert " 1 rates added" in B.describe()
+
+
+def _advance():
+    import torch
+    m = models.gene_expression((1, 1, 1, 30, 40))
+    B = BDFIntegrator(FSPMat.from_model(m, MatrixFormat.KRONECKER), rtol=1e-8, atol=1e-14)
+    p = torch.as_tensor(m.p0(), device="cuda")
+    B.init(0.0, p)
+    B.advance(1.0, p)
+    return p.cpu().numpy(), B.describe()
+
+
+def test_report_copied_instead_of_polled(cuda, tmp_path):
+    """CUFSP_BDF_SPIN=0 holds for the persistent step, too."""
+    import os
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    import numpy as np
+    root = Path(__file__).resolve().parent.parent
+    code = ("import sys; sys.path[:0] = [%r, %r]\nimport numpy as np, test_gpu_bdf_forms as t\np, d = t._advance()\n"
+            "assert d.endswith('report copied'), d\nnp.save(%r, p)" % (str(root), str(root / "tests"), str(tmp_path / "p.npy")))
+    subprocess.run([sys.executable, "-c", code], check=True, env={**os.environ, "CUFSP_BDF_SPIN": "0"})
+    p, d = _advance()
+    assert d.endswith("report polled"), d
+    assert np.array_equal(np.load(tmp_path / "p.npy"), p)
