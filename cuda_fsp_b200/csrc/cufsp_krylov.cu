@@ -228,7 +228,8 @@ __global__ void __launch_bounds__(kRedThreads) k_mupd(const MVecArgs a) {
 // vectors of U pairs, U = 2 where the window has at most four vectors (incomplete orthogonalisation),
 // whose three or four 8-byte loads of one state left the memory idle.  The update walks the vectors
 // backwards: the ends, which the dots have read last, are still in L2 (126 MB).
-// With at most four vectors the update reads the oldest with the evict-first hint: it leaves the window, and
+// Where the window is full and has at most four vectors (DROP), the update reads the oldest with the
+// evict-first hint: it leaves the window, and
 // the L2 lines it gives up keep what the generator and the next dots read (one iteration, window of 3: 5.5M
 // states 110.7 -> 107.7 us, 2.6M states 55.8 -> 53.2 us, 16.8M states 340 -> 333 us).  The dots backwards and
 // the update forwards would take 113 us at 5.5M states, stores of the generator without their hint 109.0 us.
@@ -298,7 +299,7 @@ __global__ void __launch_bounds__(kRedThreads, 3) k_mdot_pairs(const MVecArgs a)
     }
 }
 
-template <int KB, int U>
+template <int KB, int U, bool DROP>
 __global__ void __launch_bounds__(kRedThreads, 3) k_mupd_pairs(const MVecArgs a) {
     __shared__ RedSmem<1> sm;
     __shared__ double g[kMaxVec + 8];
@@ -325,7 +326,7 @@ __global__ void __launch_bounds__(kRedThreads, 3) k_mupd_pairs(const MVecArgs a)
                 for (int k = 0; k < KB; ++k) {
                     x[u][k] = make_double2(0.0, 0.0);
                     if (i >= 0 && k0 + k < a.K)
-                        x[u][k] = U == 2 && k == 0 ? __ldcs(p_first + i) : __ldg((k0 + k ? Wb + (int64_t)(k0 + k - 1) * np : p_first) + i);
+                        x[u][k] = DROP && k == 0 ? __ldcs(p_first + i) : __ldg((k0 + k ? Wb + (int64_t)(k0 + k - 1) * np : p_first) + i);
                 }
             }
 #pragma unroll
@@ -493,8 +494,9 @@ cufsp_status arnoldi_dot_update(cufsp_expv *E, double *v, int j, int istart, cud
         else if (K <= 32) k_mdot_pairs<8, 4, 1><<<g, kRedThreads, 0, st>>>(a);
         else k_mdot_pairs<8, 8, 1><<<g, kRedThreads, 0, st>>>(a);
         CUFSP_CUDA_TRY(cudaGetLastError());
-        if (K <= 4) k_mupd_pairs<4, 2><<<g, kRedThreads, 0, st>>>(a);
-        else k_mupd_pairs<8, 1><<<g, kRedThreads, 0, st>>>(a);
+        if (K <= 4 && E->iop && K == E->q_iop) k_mupd_pairs<4, 2, true><<<g, kRedThreads, 0, st>>>(a);
+        else if (K <= 4) k_mupd_pairs<4, 2, false><<<g, kRedThreads, 0, st>>>(a);
+        else k_mupd_pairs<8, 1, false><<<g, kRedThreads, 0, st>>>(a);
         CUFSP_CUDA_TRY(cudaGetLastError());
         return CUFSP_SUCCESS;
     }
