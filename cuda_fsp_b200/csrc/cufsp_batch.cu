@@ -272,9 +272,9 @@ int clusters_for(cufsp_batch *B, const BatchKernel &k, int cluster, int threads)
 // Basis vectors start on 16-byte boundaries: their stride in doubles.
 long long ld_max(const cufsp_batch *B) { return (B->n_max + 1) & ~(int64_t)1; }
 
-// Doubles of one cluster's workspace: m + 1 basis vectors, and the tables of up to 16 CTAs.
+// Doubles of one cluster's workspace: m + 1 basis vectors, and the tables that shared memory does not hold.
 long long work_stride(const cufsp_batch *B) {
-    const long long tabs = B->tab_smem ? 0 : 16LL * (B->nr + 1) * B->stride_max;
+    const long long tabs = B->tab_smem ? 0 : (long long)(B->nr + 1) * B->stride_max;
     return (B->m + 1) * ld_max(B) + ((tabs + 1) & ~1LL);
 }
 
@@ -300,7 +300,6 @@ cufsp_status launch(cufsp_batch *B, const BatchKernel &k, int cluster, int threa
     a.work = B->d_work;
     a.work_stride = work_stride(B);
     a.ld_max = (int)ld_max(B);
-    a.stride_max = B->stride_max;
     a.counter = B->d_counter;
     a.stats = B->d_stats;
     a.n_inst = n_inst;

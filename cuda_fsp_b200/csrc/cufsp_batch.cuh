@@ -61,11 +61,11 @@ struct CufspBatchArgs {
     const double *tables;    // packed factor tables
     double *p;               // packed state vectors (in: p(0), out: p(t_final))
     double *work;            // per-cluster basis workspace, work_stride doubles each
-    long long work_stride;   // >= (M + 1) ld_max, and the CTAs' tables where they are not in shared memory; even
+    long long work_stride;   // >= (M + 1) ld_max, and the cluster's tables where they are not in shared memory; even
     unsigned *counter;       // work counter (zero before the launch)
     CufspBatchStat *stats;   // per instance
     int n_inst;
-    int ld_max, stride_max;  // longest basis vector (even), largest tab_stride
+    int ld_max;              // longest basis vector (even)
     int max_steps, max_reject;
     double t_final, tol, anorm;
 };
@@ -115,8 +115,8 @@ struct Shared {
 __device__ __forceinline__ void cluster_sum1(cg::cluster_group &cl, Shared &s, double v, int &buf);
 
 // ---- generator action from per-instance tables ----------------------------------------------------
-// At the start of an instance every CTA writes its rates into tables (shared memory when they fit beside
-// the solver's state, else the cluster's workspace): gain[r][s][x_s], the factor of reaction r at the
+// At the start of an instance the rates are written into tables (every CTA its own in shared memory when they
+// fit beside the solver's state, else the cluster's CTAs one in its workspace): gain[r][s][x_s], the factor of reaction r at the
 // source state x - nu_r, 0 where that leaves the box, with the rate in the first species' factor; and
 // loss[s][x_s], the summed outflow of the reactions whose propensity depends on species s alone.  A state
 // then needs no bounds tests, conversions or factor products of its own: 5 + 16 table reads for the
@@ -217,13 +217,13 @@ __device__ __forceinline__ double apply_at(const CufspBatchInst &in, const Table
     return rho * fma(-dg, v[i], acc);
 }
 
-template <int R, int SP>
+template <int R, int SP>  // by threads `me` of `step`
 __device__ __forceinline__ void fill_tables(const CufspBatchInst &in, const double *__restrict__ tab, double *gain,
-                                            double *loss) {
+                                            double *loss, int me, int step) {
     if constexpr (R < NR) {
         if constexpr (SP < NS) {
             const double *own = tab + R * in.tab_stride + in.tab_off[SP];
-            for (int x = threadIdx.x; x < in.dims[SP]; x += T) {
+            for (int x = me; x < in.dims[SP]; x += step) {
                 if constexpr (used(R, SP)) {
                     const int y = x - nu(R, SP);
                     double g = y < 0 || y >= in.dims[SP] ? 0.0 : kind(R, SP) == 0 ? 1.0 : __ldg(own + y);
@@ -232,9 +232,9 @@ __device__ __forceinline__ void fill_tables(const CufspBatchInst &in, const doub
                 }
                 if constexpr (own_species(R) == SP) loss[in.tab_off[SP] + x] += in.coef[R] * __ldg(own + x);
             }
-            fill_tables<R, SP + 1>(in, tab, gain, loss);
+            fill_tables<R, SP + 1>(in, tab, gain, loss, me, step);
         } else {
-            fill_tables<R + 1, 0>(in, tab, gain, loss);
+            fill_tables<R + 1, 0>(in, tab, gain, loss, me, step);
         }
     }
 }
@@ -592,7 +592,7 @@ __device__ __noinline__ void pass_combine(double *v, const double *W, int ld, in
 
 // ---- one instance --------------------------------------------------------------------------
 __device__ void solve_instance(const CufspBatchArgs &a, cg::cluster_group &cl, Shared &s, double *W, double *tabs,
-                               int ld_max, int stride_max, int &buf) {
+                               int ld_max, int &buf) {
     const int n = s.in.n;
     const int nb = (int)cl.num_blocks(), rank = (int)cl.block_rank();
     const int chunk = ((n + nb - 1) / nb + 63) & ~63;
@@ -606,13 +606,19 @@ __device__ void solve_instance(const CufspBatchArgs &a, cg::cluster_group &cl, S
     const double btol = a.anorm * a.tol;
     int steps = 0, rejects = 0, matvecs = 0, status = 0;
     Tables tb;
-    {  // each CTA its own tables: behind the solver's state in shared memory, or in the cluster's workspace
-        double *gain = CUFSP_BATCH_TABSMEM ? tabs : W + (size_t)(M + 1) * ld_max + (size_t)rank * (NR + 1) * stride_max;
-        double *loss = gain + NR * s.in.tab_stride;
-        for (int x = threadIdx.x; x < s.in.tab_stride; x += T) loss[x] = 0.0;
-        __syncthreads();
-        fill_tables<0, 0>(s.in, tab, gain, loss);
-        __syncthreads();
+    {  // behind the solver's state in shared memory, or behind the basis in the cluster's workspace
+        constexpr bool OWN = CUFSP_BATCH_TABSMEM != 0;
+        const int me = OWN ? (int)threadIdx.x : rank * T + (int)threadIdx.x, step = OWN ? T : nb * T;
+        double *gain = OWN ? tabs : W + (size_t)(M + 1) * ld_max;
+        double *loss = gain + (size_t)NR * s.in.tab_stride;
+        auto sync = [&] {
+            if constexpr (OWN) __syncthreads();
+            else cl.sync();
+        };
+        for (int x = me; x < s.in.tab_stride; x += step) loss[x] = 0.0;
+        sync();
+        fill_tables<0, 0>(s.in, tab, gain, loss, me, step);
+        sync();
         tb.gain = gain;
         tb.loss = loss;
     }
@@ -801,7 +807,7 @@ extern "C" __global__ void __launch_bounds__(CUFSP_BATCH_THREADS, CUFSP_BATCH_MI
         for (int e = threadIdx.x; e < (int)(sizeof(CufspBatchInst) / sizeof(int)); e += T)
             reinterpret_cast<int *>(&s.in)[e] = reinterpret_cast<const int *>(a.inst + idx)[e];
         __syncthreads();
-        solve_instance(a, cl, s, W, reinterpret_cast<double *>(dsm + sizeof(Shared)), a.ld_max, a.stride_max, buf);
+        solve_instance(a, cl, s, W, reinterpret_cast<double *>(dsm + sizeof(Shared)), a.ld_max, buf);
         cl.sync();  // the cluster's workspace is free again
     }
 }
