@@ -284,6 +284,7 @@ cufsp_status ensure_work(cufsp_batch *B, int n_clusters) {
     if (B->d_work) cudaFree(B->d_work);
     B->d_work = nullptr;
     B->work_doubles = 0;
+    B->tuned = false;  // should the allocation fail, no shape has a workspace: the next solve chooses one anew
     CUFSP_CUDA_TRY(dev_malloc(&B->d_work, sizeof(double) * need));
     B->work_doubles = need;
     return CUFSP_SUCCESS;

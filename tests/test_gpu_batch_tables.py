@@ -39,3 +39,28 @@ def test_workspace_of_a_long_axis(cuda):
     clusters = int(re.search(r"(\d+) clusters", B.describe()).group(1))
     n, stride, nr = ms[0].n_states, 400003, ms[0].nr
     assert used <= 8 * clusters * (11 * n + (nr + 1) * stride) + (32 << 20)  # kernels and page rounding: 32 MB
+
+
+def test_solve_after_a_shape_without_workspace(cuda):
+    """set_shape that finds no memory gives the workspace of the earlier shape back: the next solve must not use
+    it, and chooses a shape that fits."""
+    import torch
+    from cuda_fsp_b200 import CufspError
+    ms = [models.toggle((699, 699)) for _ in range(40)]
+    B = BatchKrylov.from_models(ms, m=30, tol=1e-8)
+    B.set_shape(16, 512)
+    p0 = B.pack([mm.p0() for mm in ms])
+    p, q = p0.clone(), p0.clone()
+    B.solve(1e-3, p)
+    per_cluster = 8 * 31 * ms[0].n_states  # 122 MB
+    wide = int(re.search(r"(\d+) clusters", B.describe()).group(1))
+    torch.cuda.synchronize()
+    filler = torch.empty((torch.cuda.mem_get_info()[0] - 2 * per_cluster) // 8, dtype=torch.float64, device="cuda")
+    with pytest.raises(CufspError) as e:
+        B.set_shape(2, 128)  # more clusters than `wide` + 2
+    assert e.value.name == "CUFSP_ERR_ALLOC"
+    del filler
+    torch.cuda.empty_cache()
+    B.solve(1e-3, q)
+    assert int(re.search(r"(\d+) clusters", B.describe()).group(1)) >= 1 and wide + 2 < 40
+    assert (p - q).abs().sum().item() <= 1e-9
