@@ -64,7 +64,7 @@ struct PArgs {
     double *ex;                 // exchange area of this launch, all unset
     double *ex_next;            // that of the next launch, set back to unset here
     int ex_rows;                // rows of an area
-    int *err;                   // set when a wait expired
+    Waits waits;
     double *h_state;            // pinned host copy of the state block (nullable), its length and sequence word
     int words;
     unsigned *h_seq, seq;
@@ -162,9 +162,9 @@ __global__ void __launch_bounds__(NT, 1) k_arnoldi_persistent(const __grid_const
         if (!last || a.with_avnorm) {
             if constexpr (REG) {
                 double v[NS][TF];
-                bad = !gather_begin<NT, NS, TF, false>(a.terms, x, lo, len, j > 0, xs, v, a.err);
+                bad = !gather_begin<NT, NS, TF, false>(a.terms, x, lo, len, j > 0, xs, v, a.waits);
                 __syncthreads();
-                if (!gather_end<NT, NS, TN, TF>(a.terms, x, lo, len, j > 0, xs, cn, cfar, v, w, a.err)) bad = true;
+                if (!gather_end<NT, NS, TN, TF>(a.terms, x, lo, len, j > 0, xs, cn, cfar, v, w, a.waits)) bad = true;
 #pragma unroll
                 for (int s = 0; s < NS; ++s) {
                     if (tid + s * NT < len) ws[tid + s * NT] = w[s];
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(NT, 1) k_arnoldi_persistent(const __grid_const
                             sum = fma(__ldg(a.coef + (size_t)t * a.n + lo + il), v, sum);
                         }
                         if (j == 0 || !miss) break;
-                        bad = bad || wait.give_up(a.err);
+                        bad = bad || wait.give_up(a.waits);
                     } while (!bad);
                     ws[il] = sum;
                     aw2 = fma(sum, sum, aw2);
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(NT, 1) k_arnoldi_persistent(const __grid_const
             const double v = warp_sum(lane < NW ? (last ? sm.asum : sm.wsum)[lane] : 0.0);
             if (lane == 0 && (j == 0 || rows == 2)) st_relaxed(mine + (j == 0 ? 0 : pitch), settled(v));
         }
-        if (!exchange_own(a.ex, a.ex_rows, row, rows, 1, NW, j == 0, a.err)) bad = true;
+        if (!exchange_own(a.ex, a.ex_rows, row, rows, 1, NW, j == 0, a.waits)) bad = true;
         if (warp == 0) {
 #pragma unroll 1
             for (int r = lane + 1; r < rows; r += 32) {
@@ -220,13 +220,13 @@ __global__ void __launch_bounds__(NT, 1) k_arnoldi_persistent(const __grid_const
                 const int k = a.ring > 0 ? pos + a.ring * ((j - pos) / a.ring) : istart + pos;
                 const double rk = k < j ? sm.rho[k] : 0.0;
                 double v;
-                if (!exchange_total(a.ex, a.ex_rows, row, r, a.err, v)) bad = true;
+                if (!exchange_total(a.ex, a.ex_rows, row, r, a.waits, v)) bad = true;
                 sm.dot[pos] = v;
                 c[pos] = v * (rk * rk);
             }
         } else if (warp == NW - 1) {  // the norm has come earlier: its root and inverse hide behind the dots
             double v;
-            if (!exchange_total(a.ex, a.ex_rows, row, 0, a.err, v)) bad = true;
+            if (!exchange_total(a.ex, a.ex_rows, row, 0, a.waits, v)) bad = true;
             const double sn = sqrt(v);
             sm.sn = sn;
             sm.rj = sn > 0.0 ? 1.0 / sn : 0.0;
@@ -714,7 +714,7 @@ cufsp_status parnoldi_run(PArnoldi **ppa, cufsp_mat *A, const std::vector<double
     a.ex = pa->d_ex + (size_t)pa->turn * area;
     a.ex_next = pa->d_ex + (size_t)(1 - pa->turn) * area;
     a.ex_rows = pa->ex_rows;
-    a.err = err;
+    a.waits = launch_waits(err);
     a.h_state = h_state;
     a.words = words;
     a.h_seq = h_seq;

@@ -67,7 +67,7 @@ struct StepArgs {
     int ex_rows;
     double *h_out;                    // report block (pinned host or device memory) and its sequence word
     unsigned *h_seq, seq;
-    int *err;
+    Waits waits;
 };
 
 struct StepSmem {
@@ -80,8 +80,8 @@ struct StepSmem {
 };
 
 // The owners' part of an exchange, by the compute warps but the first, which publishes.
-__device__ __forceinline__ bool own(double *ex, int ex_rows, int row, int rows, int *err) {
-    return threadIdx.x >= kThreads || exchange_own(ex, ex_rows, row, rows, 1, kWarps, false, err);
+__device__ __forceinline__ bool own(double *ex, int ex_rows, int row, int rows, const Waits &waits) {
+    return threadIdx.x >= kThreads || exchange_own(ex, ex_rows, row, rows, 1, kWarps, false, waits);
 }
 
 template <int NS, int TN, int TF>
@@ -211,8 +211,8 @@ __global__ void __launch_bounds__(kThreads + 32, 1) k_bdf_step(const __grid_cons
         acc = 0.0;
         {
             double v[NS][TF];
-            if (work) bad = !gather_begin<NT, NS, TF, true>(a.terms, x, lo, len, true, xs, v, a.err);
-            if (work && !gather_end<NT, NS, TN, TF>(a.terms, x, lo, len, true, xs, cn, cf, v, q, a.err)) bad = true;
+            if (work) bad = !gather_begin<NT, NS, TF, true>(a.terms, x, lo, len, true, xs, v, a.waits);
+            if (work && !gather_end<NT, NS, TN, TF>(a.terms, x, lo, len, true, xs, cn, cf, v, q, a.waits)) bad = true;
         }
         if (J < 0) {
             if (__syncthreads_or(bad)) return;
@@ -229,10 +229,10 @@ __global__ void __launch_bounds__(kThreads + 32, 1) k_bdf_step(const __grid_cons
             block_part(0, acc);
             __syncthreads();
             if (!work) publish_part(0, 0);
-            if (!own(a.ex, a.ex_rows, row, 1, a.err)) bad = true;
+            if (!own(a.ex, a.ex_rows, row, 1, a.waits)) bad = true;
             if (!work) {
                 double v;
-                if (!exchange_total(a.ex, a.ex_rows, row, 0, a.err, v)) bad = true;
+                if (!exchange_total(a.ex, a.ex_rows, row, 0, a.waits, v)) bad = true;
                 sm.beta = sqrt(v);
                 sm.inv = 1.0 / sm.beta;
                 sm.gv[0] = sm.beta;
@@ -276,13 +276,13 @@ __global__ void __launch_bounds__(kThreads + 32, 1) k_bdf_step(const __grid_cons
                 else publish_part(0, K);
                 __syncthreads();
                 if (tid < K) st_relaxed(mine + (size_t)(row + tid) * pitch, settled(dots_sum<kLog>(sm.part, K, tid)));
-                if (!own(a.ex, a.ex_rows, row, K + 1, a.err)) bad = true;
+                if (!own(a.ex, a.ex_rows, row, K + 1, a.waits)) bad = true;
                 if (!work) {
                     double s2 = 0.0, v = 0.0;
 #pragma unroll 1
                     for (int r = lane; r <= K; r += 32) {
                         double u;
-                        if (!exchange_total(a.ex, a.ex_rows, row, r, a.err, u)) bad = true;
+                        if (!exchange_total(a.ex, a.ex_rows, row, r, a.waits, u)) bad = true;
                         if (r == K) {
                             v = u;
                         } else {
@@ -345,10 +345,10 @@ __global__ void __launch_bounds__(kThreads + 32, 1) k_bdf_step(const __grid_cons
                 block_part(1, acc);
                 __syncthreads();
                 if (!work) publish_part(1, 0);
-                if (!own(a.ex, a.ex_rows, row, 1, a.err)) bad = true;
+                if (!own(a.ex, a.ex_rows, row, 1, a.waits)) bad = true;
                 if (!work) {
                     double v;
-                    if (!exchange_total(a.ex, a.ex_rows, row, 0, a.err, v)) bad = true;
+                    if (!exchange_total(a.ex, a.ex_rows, row, 0, a.waits, v)) bad = true;
                     sm.hn = sqrt(v);
                     sm.inv = 1.0 / sm.hn;
                 }
@@ -437,10 +437,10 @@ __global__ void __launch_bounds__(kThreads + 32, 1) k_bdf_step(const __grid_cons
     block_part(0, acc);
     __syncthreads();
     if (!work) publish_part(0, 0);
-    if (!own(a.ex, a.ex_rows, row, 1, a.err)) bad = true;
+    if (!own(a.ex, a.ex_rows, row, 1, a.waits)) bad = true;
     if (!work) {
         double v;
-        if (!exchange_total(a.ex, a.ex_rows, row, 0, a.err, v)) bad = true;
+        if (!exchange_total(a.ex, a.ex_rows, row, 0, a.waits, v)) bad = true;
         sm.err = a.econst * sqrt(v);
     }
     row += 1;
@@ -488,10 +488,10 @@ __global__ void __launch_bounds__(kThreads + 32, 1) k_bdf_step(const __grid_cons
         publish_part(0, 0);
         publish_part(1, 1);
     }
-    own(a.ex, a.ex_rows, row, 2, a.err);
+    own(a.ex, a.ex_rows, row, 2, a.waits);
     if (blockIdx.x == 0 && !work) {
         double em, ep;
-        const bool ok = exchange_total(a.ex, a.ex_rows, row, 0, a.err, em) && exchange_total(a.ex, a.ex_rows, row, 1, a.err, ep);
+        const bool ok = exchange_total(a.ex, a.ex_rows, row, 0, a.waits, em) && exchange_total(a.ex, a.ex_rows, row, 1, a.waits, ep);
         row += 2;
         if (ok && teller) report(kBdfAccepted, J, err, sqrt(em), sqrt(ep));
     }
@@ -756,7 +756,6 @@ cufsp_status bdf_stepper_create(cufsp_mat *A, int maxl, cudaStream_t st, BdfStep
     a.gain = B->d_units;
     a.out = B->d_units + units;
     a.base = B->d_units + 2 * units;
-    a.err = B->d_err;
     B->used = true;  // the unit tables were built on st
     B->last = st;
     *out = B;
@@ -823,6 +822,7 @@ cufsp_status bdf_stepper_run(BdfStepper *B, const BdfStepIn &in, BdfStepOut &out
     a.h_out = in.d_out ? in.d_out : in.h_out;
     a.h_seq = in.d_out ? reinterpret_cast<unsigned *>(in.d_out + kBdfOutWords) : in.h_seq;
     a.seq = ++*in.seq;
+    a.waits = launch_waits(B->d_err);
     B->copied = in.d_out != nullptr;
     if (B->last != st) B->mixed = true;
     B->last = st;

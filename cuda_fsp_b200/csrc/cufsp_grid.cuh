@@ -8,14 +8,28 @@
 // written once per launch and set back to kUnset by an earlier launch, or in the same launch before a
 // fenced exchange.
 //
-// Waits are bounded (kWaitNs by the global timer): on expiry the error word is set, every waiting CTA
+// Waits are bounded (Waits::ns by the global timer): on expiry the error word is set, every waiting CTA
 // sees it, and all CTAs leave.
 #pragma once
 #include <cuda_runtime.h>
 
+#include <cstdlib>
+
 namespace cufsp {
 
-constexpr unsigned long long kWaitNs = 300ull * 1000 * 1000;
+// What a wait is given: its error word and its limit.
+struct Waits {
+    int *err;               // set when a wait expired
+    unsigned every;         // the limit is looked at every (every + 1) polls, a power of two
+    unsigned long long ns;
+};
+// Of a launch: 0.3 s, or CUFSP_GRID_WAIT_NS (the tests of what follows an expired wait set 0: the second poll
+// of a wait that finds nothing gives up).
+inline Waits launch_waits(int *err) {
+    const char *e = getenv("CUFSP_GRID_WAIT_NS");
+    const unsigned long long ns = e ? strtoull(e, nullptr, 10) : 300ull * 1000 * 1000;
+    return Waits{err, ns ? 127u : 0u, ns};
+}
 constexpr int kUnsetByte = 0xff;  // memset value that makes every double kUnset
 
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -52,13 +66,13 @@ __device__ __forceinline__ double settled(double v) {
 struct Patience {
     unsigned polls = 0;
     unsigned long long t0 = 0;
-    __device__ __forceinline__ bool give_up(int *err) {
-        if ((++polls & 127u) != 0) return false;
-        if (*(volatile int *)err) return true;
+    __device__ __forceinline__ bool give_up(const Waits &w) {
+        if ((++polls & w.every) != 0) return false;
+        if (*(volatile int *)w.err) return true;
         const unsigned long long t = global_ns();
-        if (polls == 128u) t0 = t;
-        else if (t - t0 > kWaitNs) {
-            atomicExch(err, 1);
+        if (polls == w.every + 1u) t0 = t;
+        else if (t - t0 >= w.ns) {
+            atomicExch(w.err, 1);
             return true;
         }
         return false;
@@ -103,7 +117,7 @@ __host__ __device__ inline int exchange_doubles(int rows, int grid) { return row
 // `row` is the number of the exchange's first row in the area, `all` the area's rows.  With `fence`,
 // what a CTA wrote and fenced before it published is visible to whoever has read a total and fenced.
 __device__ __forceinline__ bool exchange_own(double *area, int all, int row, int rows, int w0, int warps, bool fence,
-                                             int *err) {
+                                             const Waits &waits) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, G = (int)gridDim.x;
     const int pitch = exchange_pitch(G);
     bool ok = true;
@@ -124,7 +138,7 @@ __device__ __forceinline__ bool exchange_own(double *area, int all, int row, int
                 miss = miss || is_unset(v[i].x) || is_unset(v[i].y);
             }
             if (!miss) break;
-            ok = !w.give_up(err);
+            ok = !w.give_up(waits);
         } while (ok);
         double s = 0.0;
 #pragma unroll
@@ -138,11 +152,11 @@ __device__ __forceinline__ bool exchange_own(double *area, int all, int row, int
 }
 
 // Total of row `r` (< rows) of the exchange, from this CTA's copy.
-__device__ __forceinline__ bool exchange_total(const double *area, int all, int row, int r, int *err, double &v) {
+__device__ __forceinline__ bool exchange_total(const double *area, int all, int row, int r, const Waits &waits, double &v) {
     const double *p = area + (size_t)all * exchange_pitch((int)gridDim.x) + (size_t)(blockIdx.x % kCopies) * all + row + r;
     Patience w;
     for (v = ld_relaxed(p); is_unset(v); v = ld_relaxed(p))
-        if (w.give_up(err)) return false;
+        if (w.give_up(waits)) return false;
     return true;
 }
 

@@ -60,7 +60,7 @@ __device__ __forceinline__ double far_entry(const double *x, int lo, int rel, in
 // or loses (32,768 states: 5.70 and 5.50 ms), its 7 or 8 warps then poll for far entries all the earlier.
 template <int NT, int NS, int TF, bool EDGES>
 __device__ __forceinline__ bool gather_begin(const SliceTerms &a, const double *x, int lo, int len, bool poll, double *xs,
-                                             double (&v)[NS][TF], int *err) {
+                                             double (&v)[NS][TF], const Waits &waits) {
     const int tid = threadIdx.x, lane = tid & 31;
     bool ok = true;
 #pragma unroll
@@ -74,7 +74,7 @@ __device__ __forceinline__ bool gather_begin(const SliceTerms &a, const double *
         const int rel = e < a.halo ? e - a.halo : len + e - a.halo;
         double h = far_entry(x, lo, rel, a.n);
         while (poll && is_unset(h)) {
-            if (wait.give_up(err)) {
+            if (wait.give_up(waits)) {
                 ok = false;
                 break;
             }
@@ -107,7 +107,7 @@ __device__ __forceinline__ bool gather_begin(const SliceTerms &a, const double *
 template <int NT, int NS, int TN, int TF>
 __device__ __forceinline__ bool gather_end(const SliceTerms &a, const double *x, int lo, int len, bool poll,
                                            const double *xs, const double (&cn)[NS][TN], const double (&cf)[NS][TF],
-                                           double (&v)[NS][TF], double (&w)[NS], int *err) {
+                                           double (&v)[NS][TF], double (&w)[NS], const Waits &waits) {
     const int tid = threadIdx.x;
     bool ok = true;
 #pragma unroll
@@ -133,7 +133,7 @@ __device__ __forceinline__ bool gather_end(const SliceTerms &a, const double *x,
                         v[s][t] = far_entry(x, lo, tid + s * NT - a.far_shift[t], a.n);
                     }
             if (!miss) break;
-            if (wait.give_up(err)) {
+            if (wait.give_up(waits)) {
                 ok = false;
                 break;
             }
