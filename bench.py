@@ -506,9 +506,9 @@ def gradient_secondary(n_sets: int = 64, workers: int = 4, sample: int = 8) -> d
     """Gradient leg: d log L / d log theta for the 12 rates of the gene-expression model (131,072 states) from
     1,000 seeded-SSA cells at 8 log-spaced times in [1, 60], (n, c) histograms marginalised over the
     gene states, for n_sets parameter sets (rates within half a decade of nominal) at once
-    (cufsp_likelihood_grad_batched: `workers` concurrent adjoint solves, each worker's persistent
-    Arnoldi passes on an equal share of the SMs, so that one solve's passes overlap the others' host-side
-    step control).  The comparator is the same path one set at a time on `sample` of the same sets
+    (cufsp_likelihood_grad_batched: up to `workers` concurrent adjoint solves; at this size two of them run,
+    whose persistent Arnoldi passes take turns on the whole GPU, so that one solve's passes overlap the
+    other's host-side step control).  The comparator is the same path one set at a time on `sample` of the same sets
     (every n_sets/sample-th: the sets differ in cost, since the step count follows the rates), whose
     results the batched ones must match; one log-likelihood evaluation is timed beside it."""
     import torch
@@ -541,16 +541,16 @@ def gradient_secondary(n_sets: int = 64, workers: int = 4, sample: int = 8) -> d
     ev = time.perf_counter() - t0
     return {"metric": "grad logL grads/s", "workload": "gene_expression 131,072 states, 12 rates, 8 times in [1, 60], "
             f"1,000 SSA cells per time, marginalised over gene states, {n_sets} parameter sets",
-            "value": round(n_sets / batched, 3), "s_per_batch": round(batched, 3), "workers": workers,
+            "value": round(n_sets / batched, 3), "s_per_batch": round(batched, 3), "workers_asked": workers,
             "single_grads_per_s": round(len(idx) / single, 3),
             "single_sample": f"{len(idx)} of the same sets one at a time (cufsp_likelihood_grad)",
             "rel_diff_vs_single": {
                 "logL": dll, "grad": diff,
-                "note": "the workers' passes run on a quarter of the SMs (37 CTAs against 148) and round "
-                        "differently; where that flips an accept/reject decision of the Krylov step control, "
-                        "data cells whose probability is below the absolute kry_tol 1e-8 cross the 1e-44 floor "
-                        "(up to ~70 in log L each). With equal CTA counts both paths do the same arithmetic "
-                        "(test_c5_batched_gradients_equal_single_on_full_gene_box)."},
+                "note": "two workers' passes take turns on the whole GPU and do the single call's arithmetic "
+                        "(test_c5_batched_gradients_equal_single_on_full_gene_box). Smaller generators share "
+                        "the SMs and round differently; where that flips an accept/reject decision of the "
+                        "Krylov step control, data cells whose probability is below the absolute kry_tol 1e-8 "
+                        "cross the 1e-44 floor (up to ~70 in log L each)."},
             "s_per_loglik": round(ev, 3)}
 
 

@@ -56,7 +56,7 @@ struct PArgs {
     int shift[kMaxTerms];       // source index i - shift[t] (clamped)
     const double *v0;           // W_0 (the caller's vector)
     double *W;                  // W_1 .. W_{m+1}
-    double *H, *rho, *gam, *beta, *avnorm;
+    double *H, *rho, *beta, *avnorm;
     int *flag;                  // 0 ok, >0 happy breakdown at mb = flag, -1 NaN/Inf, -2 zero vector
     int mp2, m, iop, q;
     double btol;
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(NT, 1) k_arnoldi_persistent(const __grid_const
         a.ex_next[p] = unset_value();
     if (blockIdx.x == 0) {
 #pragma unroll 1
-        for (int i = tid; i < a.mp2 * (a.mp2 + 2); i += NT) a.H[i] = 0.0;  // H, rho and gam are contiguous
+        for (int i = tid; i < a.mp2 * (a.mp2 + 2); i += NT) a.H[i] = 0.0;  // H, rho and the launch sequence's gamma are contiguous
     }
 #pragma unroll 1
     for (int il = tid; il < (a.slots + 2) * a.chunk + 2 * a.terms.halo; il += NT) ws[il] = 0.0;
@@ -642,7 +642,7 @@ cudaError_t persistent_smem_attribute() {
 }  // namespace
 
 cufsp_status parnoldi_run(PArnoldi **ppa, cufsp_mat *A, const std::vector<double> &coefs, bool transpose,
-                          int64_t n, const double *v, double *W, double *H, double *rho, double *gam, double *beta,
+                          int64_t n, const double *v, double *W, double *H, double *rho, double *beta,
                           double *avnorm, int *flag, int *err, int m, int iop, int q, double btol, bool with_avnorm,
                           double *h_state, int words, unsigned *h_seq, unsigned seq, cudaStream_t st) {
     if (!*ppa) *ppa = new PArnoldi();
@@ -695,7 +695,6 @@ cufsp_status parnoldi_run(PArnoldi **ppa, cufsp_mat *A, const std::vector<double
     a.W = W;
     a.H = H;
     a.rho = rho;
-    a.gam = gam;
     a.beta = beta;
     a.avnorm = avnorm;
     a.flag = flag;

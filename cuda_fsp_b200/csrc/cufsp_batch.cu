@@ -46,7 +46,8 @@ struct BatchKernel {
 };
 
 // Instance tables (the rates times the shifted factors) of up to this size go to shared memory, behind the
-// solver's 80 KB: two CTAs per SM still fit.  Larger ones are read through L1 from the workspace.
+// solver's state: 76 KB at m = 30, so that two CTAs per SM still fit; at m = 32 it is 86 KB, and tables above
+// 26 KB leave one.  Larger tables are read through L1 from the workspace.
 constexpr int kTabSmemMax = 32 * 1024;
 
 std::mutex g_batch_mu;

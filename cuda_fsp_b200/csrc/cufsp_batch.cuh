@@ -12,9 +12,8 @@
 //    every CTA sums the partials of all CTAs in rank order -- identical, deterministic results in all
 //    CTAs, so every CTA holds the same Hessenberg matrix and takes the same step-control decisions
 //    without further communication.
-//  * Per Arnoldi iteration: the generator action w = rho_j A W_j fused with the dots of w against the
-//    basis (one pass over the own chunk), a cluster reduction, the update w -= V h fused with ||w||^2,
-//    a second cluster reduction.  The basis is stored unnormalised (v_k = rho_k W_k) as in the
+//  * Per Arnoldi iteration, over the own chunk: the generator action w = rho_j A W_j, the dots of w against
+//    the basis, a cluster reduction, the update w -= V h fused with ||w||^2, a second cluster reduction.  The basis is stored unnormalised (v_k = rho_k W_k) as in the
 //    single-instance driver.
 //  * The small (m+2)^2 exponential is Pade(13,13) with scaling and squaring (Higham 2005, the same
 //    algorithm as the host path cufsp_expm.cpp), computed by every CTA in its shared memory; the

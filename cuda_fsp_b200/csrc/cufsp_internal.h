@@ -248,7 +248,7 @@ bool parnoldi_wanted(const cufsp_mat *A, int64_t n, int m);
 bool parnoldi_size_ok(int64_t n);  // the size rule of parnoldi_wanted alone
 bool parnoldi_fits(int64_t n, int ctas);  // the slices of n states fit the shared memory of `ctas` CTAs
 cufsp_status parnoldi_run(PArnoldi **pa, cufsp_mat *A, const std::vector<double> &coefs, bool transpose,
-                          int64_t n, const double *v, double *W, double *H, double *rho, double *gam, double *beta,
+                          int64_t n, const double *v, double *W, double *H, double *rho, double *beta,
                           double *avnorm, int *flag, int *err, int m, int iop, int q, double btol, bool with_avnorm,
                           double *h_state, int words, unsigned *h_seq, unsigned seq, cudaStream_t st);
 void parnoldi_reported(PArnoldi *pa);

@@ -659,7 +659,7 @@ cufsp_status arnoldi_pass(cufsp_expv *E, double *v, cudaStream_t st, bool with_a
     const bool persistent = E->A && parnoldi_wanted(E->A, E->n, E->m);
     const bool published = persistent && pin_ready(E);  // the pass copies the state block itself
     if (persistent) {
-        s = parnoldi_run(&E->pa, E->A, E->coefs, E->transpose, E->n, v, E->W, E->ks.H, E->ks.rho, E->ks.gam,
+        s = parnoldi_run(&E->pa, E->A, E->coefs, E->transpose, E->n, v, E->W, E->ks.H, E->ks.rho,
                          E->ks.beta, E->ks.avnorm, E->ks.flag, E->ks.flag + 1, E->m, E->iop, E->q_iop, btol_eff,
                          with_avnorm, published ? tl_pin.p : nullptr, (int)(E->state_bytes / sizeof(double)), tl_pin.seq,
                          published ? ++tl_pin.n : 0, st);
@@ -706,10 +706,10 @@ cufsp_status arnoldi_pass(cufsp_expv *E, double *v, cudaStream_t st, bool with_a
     const int mp2 = m + 2;
     const double *hH = E->hstate.data();
     const double *hrho = hH + (size_t)mp2 * mp2;
-    int flag, barrier_err;
+    int flag, wait_err;
     std::memcpy(&flag, hrho + 2 * mp2 + 4, sizeof(int));
-    std::memcpy(&barrier_err, reinterpret_cast<const char *>(hrho + 2 * mp2 + 4) + sizeof(int), sizeof(int));
-    if (persistent && barrier_err)
+    std::memcpy(&wait_err, reinterpret_cast<const char *>(hrho + 2 * mp2 + 4) + sizeof(int), sizeof(int));
+    if (persistent && wait_err)
         return set_error(CUFSP_ERR_CUDA, "expv: a wait between the CTAs of the persistent Arnoldi pass expired");
     if (persistent) parnoldi_reported(E->pa);
     if (!persistent && E->A) {

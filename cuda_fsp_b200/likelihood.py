@@ -186,8 +186,9 @@ class Likelihood:
     def gradient_batched(self, coef_sets, workers: int = 4, m: int | None = None,
                          tol: float | None = None) -> tuple[np.ndarray, np.ndarray]:
         """(log L [n_sets], d log L / d log c [n_sets, n_reactions]) for many parameter sets at once
-        (cufsp_likelihood_grad_batched: `workers` concurrent adjoint solves on the GPU; on the
-        131,072-state gene model 4 workers measured fastest, against 2 and 8)."""
+        (cufsp_likelihood_grad_batched: up to `workers` concurrent adjoint solves on the GPU, each on its
+        share of the SMs; above 700 states per SM, or where a share cannot hold its part of the states, two
+        take turns on the whole GPU)."""
         c = np.ascontiguousarray(np.asarray(coef_sets, np.float64).reshape(-1, self.model.nr))
         ns = c.shape[0]
         t = np.ascontiguousarray(self.times)
