@@ -512,7 +512,8 @@ extern "C" cufsp_status cufsp_likelihood_grad_batched(const cufsp_model_desc *de
     // a share's slices of the basis would no longer fit its shared memory, and each pass takes all SMs, the
     // passes of two workers in turn (one's host work beside the other's pass).  Gradients/s of 16 sets, 4 workers
     // asked for, shares and turns: 64,800 states 5.97 and 5.11, 93,312 states (630 per SM) 4.36 and 4.21,
-    // 131,072 states (886 per SM) 2.55 and 3.11.
+    // 131,072 states (886 per SM) 2.55 and 3.11; over a short horizon 16,200 states 184 and 101, 32,768 states
+    // 142 and 70, 38,088 states 96 and 60.
     // Turns, too, where a share's two working slices would not fit its shared memory (14,256 states per CTA:
     // 32 workers have 4 CTAs each, enough for 57,024 states).
     // CUFSP_GRAD_SM_SHARE=0 or 1: always turns, shares wherever they fit.  Larger generators run `workers`

@@ -229,12 +229,14 @@ __global__ void __launch_bounds__(kRedThreads) k_mupd(const MVecArgs a) {
 // whose three or four 8-byte loads of one state left the memory idle.  The update walks the vectors
 // backwards: the ends, which the dots have read last, are still in L2 (126 MB).
 // Where the window is full and has at most four vectors (DROP), the update reads the oldest with the
-// evict-first hint: it leaves the window, and
-// the L2 lines it gives up keep what the generator and the next dots read (one iteration, window of 3: 5.5M
-// states 110.7 -> 107.7 us, 2.6M states 55.8 -> 53.2 us, 16.8M states 340 -> 333 us).  The dots backwards and
-// the update forwards would take 113 us at 5.5M states, stores of the generator without their hint 109.0 us.
-// Measured, 5.5M states, window of 3 (IOP): dots 36 -> 33.6 us, update 49 -> 38.7 us (cold L2, without the hint); 16.8M states, K = 30:
-// dots 613 us and update 621 us, 6.8 and 6.9 TB/s; a step of m = 30 there 24.38 -> 24.04 ms.
+// evict-first hint: it leaves the window, and the L2 lines it gives up keep what the generator and the next
+// dots read (one iteration, window of 3: 5.5M states 110.7 -> 107.7 us, 2.6M states 55.8 -> 53.2 us, 16.8M
+// states 340 -> 333 us).  The dots backwards and the update forwards would take 113 us at 5.5M states, stores
+// of the generator without their hint 109.0 us.
+// Measured, 5.5M states, window of 3 (IOP): dots 36 -> 33.6 us, update 49 -> 38.7 us (cold L2, without the
+// hint); 16.8M states, K = 30: dots 613 us and update 621 us, 6.8 and 6.9 TB/s.  One generator application with
+// its dots and update, 8-byte and pair kernels in turn: 5.5M states, window of 3, 126 and 106 us; 16.8M
+// states, m = 30 with full orthogonalisation, 856 and 843 us.
 template <int KG, int G, int U>
 __global__ void __launch_bounds__(kRedThreads, 3) k_mdot_pairs(const MVecArgs a) {
     constexpr int KP = KG * G;
