@@ -527,7 +527,7 @@ cufsp_status build_terms(PArnoldi *pa, cufsp_mat *A, const std::vector<double> &
     std::vector<int> rterm(nr, -1);
     std::vector<int64_t> shifts;
     for (int r = 0; r < nr; ++r) {
-        if (d[r] == 0) {  // a change of several species may make up a flat shift of 0, but never inside the box
+        if (d[r] == 0 || std::llabs(d[r]) >= n) {  // no source inside the box (shifts fit an int below), or no change
             const int *nu = m.nu.data() + (size_t)r * ns;
             if (std::all_of(nu, nu + ns, [](int v) { return v == 0; })) rterm[r] = -2;
             continue;

@@ -41,6 +41,18 @@ def test_flat_shift_zero_keeps_the_outflow(cuda, fmt):
     assert abs(float(v.sum()) - np.exp(-0.7)) <= 1e-9
 
 
+@pytest.mark.parametrize("fmt", ["KRONECKER", "HYB"])
+@pytest.mark.parametrize("nu", [4, 32768, 65536, -32768])  # flat shifts n, 2^31, 2^32 and -2^31
+def test_shift_beyond_the_box_keeps_the_outflow(cuda, fmt, nu):
+    import torch
+    m = models.mass_action((65535, 3), [[0, nu], [1, 0]], [[0, 0], [0, 0]], [0.7, 2.0])
+    p = np.zeros(m.n_states)
+    p[3::65536] = 0.25
+    v = torch.as_tensor(p, device="cuda")
+    KryExpvFSP(1.0, FSPMat.from_model(m, getattr(MatrixFormat, fmt)), v, tol=1e-10, coefs=m.coefs(0)).solve()
+    assert abs(float(v.sum()) - np.exp(-0.7)) <= 1e-9
+
+
 def test_likelihood_and_gradient(cuda):
     times = np.array([0.5, 1.5])
     plain = models.mass_action(BOX, NU, ORDERS, RATES)
