@@ -27,7 +27,7 @@ struct Waits {
 // of a wait that finds nothing gives up).
 inline Waits launch_waits(int *err) {
     const char *e = getenv("CUFSP_GRID_WAIT_NS");
-    const unsigned long long ns = e ? strtoull(e, nullptr, 10) : 300ull * 1000 * 1000;
+    const unsigned long long ns = e && *e ? strtoull(e, nullptr, 10) : 300ull * 1000 * 1000;
     return Waits{err, ns ? 127u : 0u, ns};
 }
 constexpr int kUnsetByte = 0xff;  // memset value that makes every double kUnset
