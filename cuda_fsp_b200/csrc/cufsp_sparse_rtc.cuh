@@ -16,6 +16,14 @@
 // pair are issued before the first use (memory-level parallelism), and the table rows use the
 // default L2 policy, so that the shifted re-read of a row -- by the CTA |d_r| states away -- hits L2
 // instead of DRAM; y is written with the streaming policy.
+//
+// Registers limit an SM to 16 warps, whose loads of one chunk of reactions do not cover the DRAM latency:
+// a CTA therefore first asks L2 for all rows of its tile, one bulk prefetch per row by one thread each
+// (row r where it is first touched: at the source when the source lies ahead).  9 reactions: 160 x 151 x
+// 132 states 61.7 -> 59.7 us (63.2 -> 63.0 us after another generator), 256^3 275 -> 271 us; 12 reactions,
+// 0.9M states 25.9 -> 24.9 us.  Asking for
+// the tile after that, or the next two, costs more than it hides (61.0, 63.6 us; 312, 333 us): the rows
+// that are read again at their sources leave L2 sooner.
 #ifndef CUFSP_SPARSE_RTC_CUH
 #define CUFSP_SPARSE_RTC_CUH
 
@@ -147,6 +155,27 @@ __device__ __forceinline__ void all_reactions(const CufspSparseRtcArgs &a, const
     }
 }
 
+// Prefetch of [p, p + count) doubles into L2, cut to the vector's end and to 16-byte boundaries (p is one).
+__device__ __forceinline__ void prefetch_rows(const double *row, long long first, int count) {
+    first &= ~1LL;
+    const long long left = (N - first) & ~1LL;
+    const long long take = left < count ? left : count;
+    if (take > 0)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(row + first), "r"((unsigned)(take * 8)) : "memory");
+}
+
+// How far ahead of a state its row of reaction r (r < NR), x (NR) or y (NR + 1) is first touched.
+__device__ __forceinline__ long long first_touch(int r) {
+    long long ahead = 0, most = 0;
+#pragma unroll
+    for (int q = 0; q < NR; ++q) {
+        const long long d = shift(q) < 0 ? -shift(q) : 0;
+        if (q == r) ahead = d;
+        most = d > most ? d : most;
+    }
+    return r == NR ? most : ahead;
+}
+
 template <bool ACCUM>
 __device__ __forceinline__ void sparse_mv(const CufspSparseRtcArgs &a, const double *__restrict__ x,
                                           double *__restrict__ y) {
@@ -154,9 +183,17 @@ __device__ __forceinline__ void sparse_mv(const CufspSparseRtcArgs &a, const dou
     const double alpha = a.d_alpha ? __ldg(a.d_alpha) : 1.0;
     const long long first = a.i_begin & ~1LL;
     const long long pairs = (a.i_end - first + 1) >> 1;
+    const int me = (int)threadIdx.x;
+    const double *ahead_row = nullptr;  // this thread's row to prefetch
+    long long ahead = 0;
+    if (N % 2 == 0 && me < NR + (ACCUM ? 2 : 1)) {
+        ahead_row = me < NR ? a.P + (long long)me * N : me == NR ? x : y;
+        ahead = first_touch(me) - 2 * me;
+    }
     for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < pairs;
          k += (long long)gridDim.x * blockDim.x) {
         const long long i = first + 2 * k;
+        if (ahead_row) prefetch_rows(ahead_row, i + ahead, 2 * (int)blockDim.x);
         const bool pair = i + 1 < N;  // the last state of an odd-length vector is alone
         double2 xv, yv = make_double2(0.0, 0.0);
         if (pair) {
